@@ -34,9 +34,10 @@ _I64 = C.c_int64
 
 
 def build(ref: bool = True) -> None:
-    """Builds liboracle.so, and the reference libraries when the tree exists."""
+    """Builds liboracle.so, and the reference libraries when the tree holds
+    the reference's sources (it may be absent or an empty folder)."""
     targets = ["oracle"]
-    if ref and REFERENCE_TREE.is_dir():
+    if ref and (REFERENCE_TREE / "Pattern" / "Indexer.cpp").is_file():
         targets.append("ref")
     subprocess.run(["make", "-s", "-C", str(HERE), f"REF={REFERENCE_TREE}", *targets], check=True)
 
