@@ -21,21 +21,8 @@ __device__ __forceinline__ uint32_t digits(const uint8_t* sq, int n, uint32_t pl
     return idx;
 }
 
-// A row's cells as a digit board in shared memory: board[t * STRIDE] =
-// cell(pos, t) for the 64 squares, one byte each.  With STRIDE the CTA's
-// thread count and board = base + threadIdx.x, a warp's 32 rows sit in 32
-// consecutive bytes of every square's line: reads and writes of one square
-// by a warp touch 8 words, without bank conflicts.
-template <int STRIDE>
-__device__ __forceinline__ void fill_board(uint8_t* board, uint32_t plo, uint32_t phi, uint32_t olo, uint32_t ohi)
-{
-#pragma unroll
-    for (int t = 0; t < 32; t++) {
-        board[t * STRIDE] = static_cast<uint8_t>(((plo >> t) & 1u) | (((olo >> t) & 1u) << 1));
-        board[(t + 32) * STRIDE] = static_cast<uint8_t>(((phi >> t) & 1u) | (((ohi >> t) & 1u) << 1));
-    }
-}
-
+// The digits of a square list read from a row's digit board in shared
+// memory: board[t * STRIDE] = cell(pos, t) for the 64 squares, one byte each.
 template <int STRIDE>
 __device__ __forceinline__ uint32_t board_digits(const uint8_t* sq, int n, const uint8_t* board)
 {
@@ -71,30 +58,12 @@ __device__ __forceinline__ uint32_t eval_slot(const Instance& in, const uint32_t
                         [&](const uint8_t* sq, int n) { return digits(sq, n, plo, phi, olo, ohi); });
 }
 
-// eval_slot from the row's digit board (fill_board), every kind inlined.
+// eval_slot from the row's digit board.
 template <int STRIDE>
 __device__ __forceinline__ uint32_t eval_slot_board_all(const Instance& in, const uint32_t* __restrict__ tables,
                                                         const uint8_t* board)
 {
     return combine_slot(in, tables, [&](const uint8_t* sq, int n) { return board_digits<STRIDE>(sq, n, board); });
-}
-
-template <int STRIDE>
-__device__ __noinline__ uint32_t eval_slot_board_other(const Instance& in, const uint32_t* __restrict__ tables,
-                                                       const uint8_t* board)
-{
-    return eval_slot_board_all<STRIDE>(in, tables, board);
-}
-
-// The same for callers that unroll it over a pattern's slots: only the
-// direct kind (every instance of the expanded mode) is inlined, as the other
-// kinds' code would not fit the instruction cache beside it.
-template <int STRIDE>
-__device__ __forceinline__ uint32_t eval_slot_board(const Instance& in, const uint32_t* __restrict__ tables,
-                                                    const uint8_t* board)
-{
-    if (in.kind == kDirect) return in.offset + board_digits<STRIDE>(in.sq[0], in.n0, board);
-    return eval_slot_board_other<STRIDE>(in, tables, board);
 }
 
 }  // namespace cas

@@ -5,12 +5,22 @@
 
 #include "common.cuh"
 #include "patterns.h"
+#include "tile_index.h"
 
 namespace cas {
 
+// A pattern set on the device: one block that holds every array.
 struct DevicePatterns {
+    void* block = nullptr;
     Instance* instances = nullptr;
     uint32_t* tables = nullptr;
+    // the matrix form (chunks == 0: a digit list is too long for it)
+    uint32_t* tiles = nullptr;
+    IndexUnit* units = nullptr;
+    int32_t* chunk_unit = nullptr;
+    int32_t* chunk_tile = nullptr;
+    int chunks = 0;
+    size_t tile_bytes = 0;  // shared memory of the largest chunk
     int k = 0;
     int64_t cols = 0;
 };
