@@ -2,11 +2,10 @@
 // per-block column sort for the transposed copy, chunk pointers, diag(A'A))
 // and the two products.  See fast.cuh for the layout.
 //
-// A x   one CTA per row block (1024 threads, 16 rows each).  For every pattern
-//       the CTA copies that pattern's slice of x (up to 224 KB) into shared
-//       memory and every thread gathers its rows' entries from there; the
-//       uint16 index stream is read once, coalesced (16 B per row and
-//       pattern).  HBM traffic: 2 B per entry + the output.
+// A x   one row a thread, its index words (2 B per entry, 16 B per row and
+//       pattern) loaded first, then its entries of x gathered: from a table
+//       in shared memory for the patterns whose slices fit one, through L1
+//       and L2 for the others.  HBM traffic: 2 B per entry + the output.
 // A'y   one CTA per work item (a column chunk of one pattern x a range of row
 //       blocks).  Per block the CTA stages y's block slice in shared memory,
 //       streams the chunk's column-sorted entries (4 B each, coalesced),
@@ -575,31 +574,6 @@ __device__ __forceinline__ void gather_row(const uint16_t* __restrict__ src, int
     }
 }
 
-// One index word (two 16-bit columns) of a row gathered into acc.
-template <typename T, bool ALL_IN>
-__device__ __forceinline__ void gather_word(uint32_t wd, const T* __restrict__ table, const T* __restrict__ xg,
-                                            int cap, typename AccOf<T>::type& acc)
-{
-    using Acc = typename AccOf<T>::type;
-    const int c0 = static_cast<int>(wd & 0xFFFFu), c1 = static_cast<int>(wd >> 16);
-    acc += static_cast<Acc>(ALL_IN || c0 < cap ? table[c0] : __ldg(xg + c0));
-    acc += static_cast<Acc>(ALL_IN || c1 < cap ? table[c1] : __ldg(xg + c1));
-}
-
-// Scalar stores of one 16-byte vector (the destination need not be aligned).
-__device__ __forceinline__ void store_vec(float* d, uint4 u)
-{
-    d[0] = __uint_as_float(u.x);
-    d[1] = __uint_as_float(u.y);
-    d[2] = __uint_as_float(u.z);
-    d[3] = __uint_as_float(u.w);
-}
-__device__ __forceinline__ void store_vec(double* d, uint4 u)
-{
-    d[0] = __hiloint2double(static_cast<int>(u.y), static_cast<int>(u.x));
-    d[1] = __hiloint2double(static_cast<int>(u.w), static_cast<int>(u.z));
-}
-
 // Asks L2 to fetch [p, p + bytes) (the 16-byte words wholly inside it), in
 // 4 KB bulk prefetches spread over the CTA's threads.  A hint: the data is
 // read later with ordinary loads.
@@ -612,67 +586,6 @@ __device__ __forceinline__ void prefetch_l2(const void* p, int64_t bytes)
          c += static_cast<uintptr_t>(blockDim.x) * 4096) {
         const unsigned n = static_cast<unsigned>(min(static_cast<uint64_t>(e - c), static_cast<uint64_t>(4096)));
         asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(c), "r"(n) : "memory");
-    }
-}
-
-// Copies a pattern's slice of x (cap entries) into shared memory with
-// 16-byte loads, several in flight per thread.
-template <typename T>
-__device__ __forceinline__ void load_table(T* __restrict__ table, const T* __restrict__ xg, int cap)
-{
-    constexpr int kPer = 16 / sizeof(T);
-    const int mis = static_cast<int>((reinterpret_cast<uintptr_t>(xg) & 15) / sizeof(T));
-    const int head = min(cap, mis ? kPer - mis : 0);
-    if (static_cast<int>(threadIdx.x) < head) table[threadIdx.x] = xg[threadIdx.x];
-    const int nvec = (cap - head) / kPer;
-    const uint4* src = reinterpret_cast<const uint4*>(xg + head);
-    T* dst = table + head;
-    for (int v0 = threadIdx.x; v0 < nvec; v0 += 4 * blockDim.x) {
-        uint4 u[4];
-#pragma unroll
-        for (int k = 0; k < 4; k++) {
-            const int v = v0 + k * blockDim.x;
-            if (v < nvec) u[k] = __ldg(src + v);
-        }
-#pragma unroll
-        for (int k = 0; k < 4; k++) {
-            const int v = v0 + k * blockDim.x;
-            if (v < nvec) store_vec(dst + v * kPer, u[k]);
-        }
-    }
-    const int done = head + nvec * kPer;
-    for (int i = done + threadIdx.x; i < cap; i += blockDim.x) table[i] = xg[i];
-}
-
-// Rows of one 8-slot pattern segment (the expanded layout): each thread owns
-// ROWS rows (stride kAxThreads); the 16-byte index word of row j+AHEAD is
-// loaded while row j is gathered, so AHEAD loads per thread stay in flight.
-template <typename T, bool ALL_IN, int ROWS, int AHEAD>
-__device__ __forceinline__ void gather_segment8(const uint16_t* __restrict__ base, int nb,
-                                                const T* __restrict__ table, const T* __restrict__ xg, int cap,
-                                                typename AccOf<T>::type (&acc)[ROWS])
-{
-    uint4 w[AHEAD];
-#pragma unroll
-    for (int j = 0; j < AHEAD; j++) {
-        const int r = threadIdx.x + j * kAxThreads;
-        w[j] = r < nb ? *reinterpret_cast<const uint4*>(base + static_cast<int64_t>(r) * 8) : make_uint4(0, 0, 0, 0);
-    }
-#pragma unroll
-    for (int j = 0; j < ROWS; j++) {
-        const uint4 cur = w[j % AHEAD];
-        if (j + AHEAD < ROWS) {
-            const int rn = threadIdx.x + (j + AHEAD) * kAxThreads;
-            w[j % AHEAD] = rn < nb ? *reinterpret_cast<const uint4*>(base + static_cast<int64_t>(rn) * 8)
-                                   : make_uint4(0, 0, 0, 0);
-        }
-        const int r = threadIdx.x + j * kAxThreads;
-        if (r < nb) {
-            gather_word<T, ALL_IN>(cur.x, table, xg, cap, acc[j]);
-            gather_word<T, ALL_IN>(cur.y, table, xg, cap, acc[j]);
-            gather_word<T, ALL_IN>(cur.z, table, xg, cap, acc[j]);
-            gather_word<T, ALL_IN>(cur.w, table, xg, cap, acc[j]);
-        }
     }
 }
 
@@ -727,59 +640,167 @@ __host__ __device__ __forceinline__ int unit_splits(int64_t units, int64_t ctas,
     return static_cast<int>(k < 1 ? 1 : (k > cap ? cap : k));
 }
 
-// ALL8: every pattern has 8 slots (the expanded layout), so only the
-// pipelined 8-slot path is compiled in.
-// A work unit is one of a block's row splits (a CTA stages x's pattern
-// slices once per unit, so splits pay only when units are few).  part
-// (optional) receives one compensated partial of ||y||^2 per unit, so that
-// the norms of the problems of a batched layout can be summed apart.
-// Blocks of problems whose pdone flag is set are skipped (partials 0).
-// Without act: units (block, split) for every block, `split` splits each,
-// partials [block][split].  With act: the listed problems' blocks only,
-// split for `ctas` CTAs, partials [block][kAxSplitMax] (splits past the one
-// in use written 0); a split of kAxSplitMax is left to
-// fast_spmv_direct_kernel.
-// ROWS: rows per thread (a unit holds at most kAxThreads * ROWS rows: a
-// whole block), AHEAD: index loads in flight per thread.
-template <typename T, typename Y, int MODE, bool ALL8, int ROWS = kAxRows, int AHEAD = kAxAhead>
-__global__ void __launch_bounds__(kAxThreads, 1) fast_spmv_kernel(FastGeometry g, const uint16_t* __restrict__ a16,
-                                                                   const T* __restrict__ x, Y* __restrict__ y,
-                                                                   const double* __restrict__ b,
-                                                                   const double* __restrict__ coef,
-                                                                   double* __restrict__ part,
-                                                                   const int* __restrict__ done,
-                                                                   const int* __restrict__ pdone,
-                                                                   const FastActive* __restrict__ act, int split,
-                                                                   int ctas)
+// The index words of one row of a pattern (slots 16-bit columns).  STREAM:
+// past L1, whose lines stay with x.
+template <bool STREAM>
+__device__ __forceinline__ uint4 load_words(const uint16_t* __restrict__ src, int slots)
+{
+    uint4 w = make_uint4(0, 0, 0, 0);
+    if (slots == 8) {
+        if (STREAM)
+            asm volatile("ld.global.nc.L1::no_allocate.v4.u32 {%0, %1, %2, %3}, [%4];"
+                         : "=r"(w.x), "=r"(w.y), "=r"(w.z), "=r"(w.w)
+                         : "l"(src));
+        else
+            w = *reinterpret_cast<const uint4*>(src);
+    } else if (slots == 4) {
+        if (STREAM) {
+            asm volatile("ld.global.nc.L1::no_allocate.v2.u32 {%0, %1}, [%2];" : "=r"(w.x), "=r"(w.y) : "l"(src));
+        } else {
+            const uint2 u = *reinterpret_cast<const uint2*>(src);
+            w.x = u.x, w.y = u.y;
+        }
+    } else if (slots == 2) {
+        w.x = *reinterpret_cast<const uint32_t*>(src);
+    } else {
+        w.x = *src;
+    }
+    return w;
+}
+
+// The entries of a row's words gathered from src (x or a table of it) into
+// acc, in slot order.
+template <typename T, bool ALL8, bool SHARED>
+__device__ __forceinline__ void gather_words(const uint4& u, int slots, const T* __restrict__ src,
+                                             typename AccOf<T>::type& acc)
+{
+    using Acc = typename AccOf<T>::type;
+    const uint32_t w[4] = {u.x, u.y, u.z, u.w};
+#pragma unroll
+    for (int s = 0; s < 8; s++) {
+        if (ALL8 || s < slots) {
+            const uint32_t c = (s & 1) ? w[s >> 1] >> 16 : w[s >> 1] & 0xFFFFu;
+            acc += static_cast<Acc>(SHARED ? src[c] : __ldg(src + c));
+        }
+    }
+}
+
+constexpr int kRowPatterns = 8;  // patterns whose index words a thread holds at once
+
+// Row r of block blk times x: every index word first, then the gathers, so
+// that they are in flight together.  TABLE: the patterns of tab have their
+// slice of x in table.
+template <typename T, bool ALL8, bool TABLE>
+__device__ __forceinline__ typename AccOf<T>::type row_sum(const FastGeometry& g, const uint16_t* __restrict__ a16,
+                                                           int64_t blk, int r, const T* __restrict__ x,
+                                                           const FastTable& tab, const T* __restrict__ table)
+{
+    const uint16_t* bp = a16 + blk * static_cast<int64_t>(kBlockRows) * g.k;
+    const int pad = static_cast<int>(g.padded_rows(blk));
+    typename AccOf<T>::type acc = 0;
+    for (int p0 = 0; p0 < g.npat; p0 += kRowPatterns) {
+        uint4 w[kRowPatterns];
+#pragma unroll
+        for (int i = 0; i < kRowPatterns; i++) {
+            const int p = p0 + i;
+            if (p < g.npat) {
+                const int ns = ALL8 ? 8 : g.slots[p];
+                w[i] = load_words<TABLE>(bp + pad * g.slot0[p] + r * ns, ns);
+            }
+        }
+#pragma unroll
+        for (int i = 0; i < kRowPatterns; i++) {
+            const int p = p0 + i;
+            if (p < g.npat) {
+                const int ns = ALL8 ? 8 : g.slots[p];
+                if (TABLE && tab.base[p] >= 0)
+                    gather_words<T, ALL8, true>(w[i], ns, table + tab.base[p], acc);
+                else
+                    gather_words<T, ALL8, false>(w[i], ns, x + g.off[p], acc);
+            }
+        }
+    }
+    return acc;
+}
+
+// The value of a row from its product v (MODE as fast_spmv's mode), stored;
+// returns the stored value.
+template <typename Y, int MODE>
+__device__ __forceinline__ double store_row(double v, Y* __restrict__ y, const double* __restrict__ b, double c,
+                                            int64_t row)
+{
+    if (MODE == 1) v = static_cast<double>(y[row]) * -c + v;
+    if (MODE == 2) v = (b ? b[row] : 0.0) - v;
+    const Y yv = static_cast<Y>(v);
+    y[row] = yv;
+    return static_cast<double>(yv);
+}
+
+// A x with the slices of x that fit kept in shared memory (FastTable: the
+// patterns with the most entries a row per column first) and the others
+// gathered through L1 and L2.  One CTA per SM runs over a contiguous share
+// of the rows, one row a thread; the table is staged once per CTA (once per
+// problem of a batch), so nothing waits on a barrier between rows.
+//
+// Bound by the gathers: 32 random words of shared memory take 3.5 wavefronts,
+// the same through L1 about 8 tag wavefronts at a 79 % hit rate.  The table
+// ends at 140 KB because L1 holds the other patterns' popular columns: on the
+// 8-pattern expanded set, 610 blocks, FP32, tables of 0, 64, 115, 195 and 224
+// KB gave 744, 629, 543, 630 and 630 us (FP64 876, 870, 862, 1015, 1590), and
+// keeping the index words out of L1 another 3 to 7 % (without a table, where
+// L1 is large, 5 % the other way).
+//
+// The kernel before this one staged every pattern's slice for every block of
+// rows (42 us of the 143 us a block took: 665 KB a block and 16 barriers).
+// us before and now, FP32 / FP64:
+//   8 patterns expanded   200 blocks 262 / 461 -> 192 / 294   610: 625 / 1136 -> 524 / 878
+//   8 patterns reference  200 blocks 330 / 420 -> 136 / 166   610: 781 / 1032 -> 371 / 463
+// Up to kAxDirectBlocks blocks the rows are done before a table pays (8
+// patterns expanded, FP32, us without and with it: 16 blocks 26.8 and 28.9,
+// 48 64.1 and 64.0, 74 92.7 and 83).
+//
+// A unit is 1/kAxTableSplit of a block.  part (optional): compensated
+// partials of ||y||^2, one per CTA without act, else per unit laid out
+// [block][kAxSplitMax] (the rest 0).  With act only the listed problems'
+// blocks run, and none when fast_spmv_direct_kernel's launch does them.
+template <typename T, typename Y, int MODE, bool ALL8>
+__global__ void __launch_bounds__(kAxThreads, 1) fast_spmv_table_kernel(FastGeometry g, FastTable tab,
+                                                                         const uint16_t* __restrict__ a16,
+                                                                         const T* __restrict__ x, Y* __restrict__ y,
+                                                                         const double* __restrict__ b,
+                                                                         const double* __restrict__ coef,
+                                                                         double* __restrict__ part,
+                                                                         const int* __restrict__ done,
+                                                                         const int* __restrict__ pdone,
+                                                                         const FastActive* __restrict__ act)
 {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     T* table = reinterpret_cast<T*>(smem_raw);
     __shared__ double red[64];
     __shared__ int pref[kMaxProblems + 1];
     if (done && *(volatile const int*)done) return;
-    constexpr int kCap = sizeof(T) == 4 ? kTable32 : kTable64;
-    using Acc = typename AccOf<T>::type;
     const double c = MODE == 1 ? *coef : 0.0;
-    int S = split, stride = split;
-    int64_t units = g.nblocks * split;
+    int64_t nblk = g.nblocks;
     if (act) {
-        const int nblk = active_prefix(act, pref, [&](int q) { return g.pblk0[q + 1] - g.pblk0[q]; });
-        S = unit_splits(nblk, ctas, kAxSplitMax);
-        stride = kAxSplitMax;
-        units = static_cast<int64_t>(nblk) * S;
+        nblk = active_prefix(act, pref, [&](int q) { return g.pblk0[q + 1] - g.pblk0[q]; });
+        if (nblk <= kAxDirectBlocks) return;
     }
-    if (act && S == kAxSplitMax) return;  // few rows per unit: fast_spmv_direct_kernel's launch
-    for (int64_t u = blockIdx.x; u < units; u += gridDim.x) {
-        const int sp = static_cast<int>(u % S);
-        int64_t blk = u / S;
+    const int64_t units = nblk * kAxTableSplit;
+    const int64_t u0 = units * blockIdx.x / gridDim.x, u1 = units * (blockIdx.x + 1) / gridDim.x;
+    int staged = -1;  // problem whose x the table holds
+    Comp mine;
+    for (int64_t u = u0; u < u1; u++) {
+        const int sp = static_cast<int>(u % kAxTableSplit);
+        int64_t blk = u / kAxTableSplit;
         if (act) {
             const int i = static_cast<int>(blk);
             const int slot = active_slot(pref, act->n, i);
             blk = g.pblk0[act->list[slot]] + (i - pref[slot]);
         }
         const int q = g.prob_of_block(blk);
-        double* pu = part ? part + 2 * (blk * stride + sp) : nullptr;
-        if (pu && sp == 0 && static_cast<int>(threadIdx.x) < 2 * (stride - S)) pu[2 * S + threadIdx.x] = 0;
+        double* pu = part && act ? part + 2 * (blk * kAxSplitMax + sp) : nullptr;
+        if (pu && sp == 0 && static_cast<int>(threadIdx.x) < 2 * (kAxSplitMax - kAxTableSplit))
+            pu[2 * kAxTableSplit + threadIdx.x] = 0;
         if (pdone && pdone[q]) {
             if (pu && threadIdx.x == 0) {
                 pu[0] = 0;
@@ -787,56 +808,26 @@ __global__ void __launch_bounds__(kAxThreads, 1) fast_spmv_kernel(FastGeometry g
             }
             continue;
         }
-        const int rows_b = static_cast<int>(g.block_rows(blk));
-        const int r0 = static_cast<int>(static_cast<int64_t>(rows_b) * sp / S);
-        const int nb = static_cast<int>(static_cast<int64_t>(rows_b) * (sp + 1) / S) - r0;
-        const int64_t row0 = g.block_row0(blk) + r0;
         const T* xq = x + q * g.pcols;
-        Comp mine;
-        Acc acc[ROWS];
-#pragma unroll
-        for (int j = 0; j < ROWS; j++) acc[j] = 0;
-        // the index stream of a pattern is fetched into L2 one phase ahead,
-        // so that HBM keeps streaming while x's next slice is staged
-        prefetch_l2(a16 + g.seg(blk, 0) + static_cast<int64_t>(r0) * g.slots[0],
-                    static_cast<int64_t>(nb) * g.slots[0] * 2);
-        for (int p = 0; p < g.npat; p++) {
-            const int cap = min(g.space[p], kCap);
-            const T* xg = xq + g.off[p];
+        if (q != staged) {
             __syncthreads();
-            load_table<T>(table, xg, cap);
-            __syncthreads();
-            if (p + 1 < g.npat)
-                prefetch_l2(a16 + g.seg(blk, p + 1) + static_cast<int64_t>(r0) * g.slots[p + 1],
-                            static_cast<int64_t>(nb) * g.slots[p + 1] * 2);
-            const int ns = g.slots[p];
-            const uint16_t* base = a16 + g.seg(blk, p) + static_cast<int64_t>(r0) * ns;
-            const bool all_in = g.space[p] <= kCap;
-            if (ALL8 || ns == 8) {
-                if (all_in)
-                    gather_segment8<T, true, ROWS, AHEAD>(base, nb, table, xg, cap, acc);
-                else
-                    gather_segment8<T, false, ROWS, AHEAD>(base, nb, table, xg, cap, acc);
-            } else if (!ALL8) {
-#pragma unroll
-                for (int j = 0; j < ROWS; j++) {
-                    const int r = threadIdx.x + j * kAxThreads;
-                    if (r < nb) gather_row<T>(base + static_cast<int64_t>(r) * ns, ns, table, xg, cap, all_in, acc[j]);
-                }
+            for (int p = 0; p < g.npat; p++) {
+                if (tab.base[p] < 0) continue;
+                T* dst = table + tab.base[p];
+                const T* src = xq + g.off[p];
+#pragma unroll 8
+                for (int i = threadIdx.x; i < g.space[p]; i += kAxThreads) dst[i] = __ldg(src + i);
             }
+            __syncthreads();
+            staged = q;
         }
-#pragma unroll
-        for (int j = 0; j < ROWS; j++) {
-            const int r = threadIdx.x + j * kAxThreads;
-            if (r < nb) {
-                const int64_t row = row0 + r;
-                double v = static_cast<double>(acc[j]);
-                if (MODE == 1) v = static_cast<double>(y[row]) * -c + v;
-                if (MODE == 2) v = (b ? b[row] : 0.0) - v;
-                const Y yv = static_cast<Y>(v);
-                y[row] = yv;
-                mine.add(static_cast<double>(yv) * static_cast<double>(yv));
-            }
+        const int rows_b = static_cast<int>(g.block_rows(blk));
+        const int r0 = rows_b * sp / kAxTableSplit, nb = rows_b * (sp + 1) / kAxTableSplit - r0;
+        if (static_cast<int>(threadIdx.x) < nb) {
+            const int r = r0 + threadIdx.x;
+            const double v = static_cast<double>(row_sum<T, ALL8, true>(g, a16, blk, r, xq, tab, table));
+            const double yv = store_row<Y, MODE>(v, y, b, c, g.block_row0(blk) + r);
+            mine.add(yv * yv);
         }
         if (pu) {
             const Comp r = block_sum_comp<kAxThreads>(mine, red);
@@ -844,21 +835,25 @@ __global__ void __launch_bounds__(kAxThreads, 1) fast_spmv_kernel(FastGeometry g
                 pu[0] = r.s;
                 pu[1] = r.c;
             }
+            mine = Comp{};
+        }
+    }
+    if (part && !act) {
+        const Comp r = block_sum_comp<kAxThreads>(mine, red);
+        if (threadIdx.x == 0) {
+            part[2 * blockIdx.x] = r.s;
+            part[2 * blockIdx.x + 1] = r.c;
         }
     }
 }
 
-constexpr int kDirectPatterns = 8;  // most 8-slot patterns of the direct A x's unrolled path
-
-// A x over units of at most kAxDirectRows rows (a block split kAxSplitMax
-// ways) without staging x: one thread per row gathers its entries through
-// L1/L2 in pattern and slot order, the order of the staged kernel, so both
-// give the same values.  Few remaining rows (the last small problems of a
-// batch, a small fit) are not worth staging every x slice per CTA.  Without
-// act it runs when the host chose kAxSplitMax splits; with act it decides on
-// the device, as the staged kernel (launched beside it) does with the same
-// `ctas`, and exactly one of the two does the work.  Partials as the staged
-// kernel's with stride kAxSplitMax.
+// A x on at most kAxDirectBlocks blocks (a small fit, the last small problems
+// of a batch): units of 1/kAxSplitMax of a block, one row a thread, all
+// gathers through L1 and L2, in the order of the table kernel, so both give
+// the same values.  So few rows are done before a table would be staged.
+// Without act it runs when the host chose it; with act it decides on the
+// device, as the table kernel (launched beside it) does, and exactly one of
+// the two does the work.  Partials [block][kAxSplitMax].
 template <typename T, typename Y, int MODE, bool ALL8>
 __global__ void __launch_bounds__(kAxDirectRows) fast_spmv_direct_kernel(FastGeometry g,
                                                                          const uint16_t* __restrict__ a16,
@@ -868,17 +863,16 @@ __global__ void __launch_bounds__(kAxDirectRows) fast_spmv_direct_kernel(FastGeo
                                                                          double* __restrict__ part,
                                                                          const int* __restrict__ done,
                                                                          const int* __restrict__ pdone,
-                                                                         const FastActive* __restrict__ act, int ctas)
+                                                                         const FastActive* __restrict__ act)
 {
     __shared__ double red[64];
     __shared__ int pref[kMaxProblems + 1];
     if (done && *(volatile const int*)done) return;
-    using Acc = typename AccOf<T>::type;
     const double c = MODE == 1 ? *coef : 0.0;
     int64_t nblk = g.nblocks;
     if (act) {
         nblk = active_prefix(act, pref, [&](int q) { return g.pblk0[q + 1] - g.pblk0[q]; });
-        if (unit_splits(nblk, ctas, kAxSplitMax) != kAxSplitMax) return;  // the staged kernel's work
+        if (nblk > kAxDirectBlocks) return;  // the table kernel's work
     }
     const int64_t units = nblk * kAxSplitMax;
     for (int64_t u = blockIdx.x; u < units; u += gridDim.x) {
@@ -899,45 +893,13 @@ __global__ void __launch_bounds__(kAxDirectRows) fast_spmv_direct_kernel(FastGeo
             continue;
         }
         const int rows_b = static_cast<int>(g.block_rows(blk));
-        const int r0 = static_cast<int>(static_cast<int64_t>(rows_b) * sp / kAxSplitMax);
-        const int nb = static_cast<int>(static_cast<int64_t>(rows_b) * (sp + 1) / kAxSplitMax) - r0;
-        const T* xq = x + q * g.pcols;
+        const int r0 = rows_b * sp / kAxSplitMax, nb = rows_b * (sp + 1) / kAxSplitMax - r0;
         Comp mine;
-        const int r = threadIdx.x;
-        if (r < nb) {
-            Acc acc = 0;
-            if (ALL8) {
-                // up to kDirectPatterns patterns of 8 slots: every index word
-                // first, then all gathers, so that they are in flight together
-                uint4 w[kDirectPatterns];
-#pragma unroll
-                for (int p = 0; p < kDirectPatterns; p++)
-                    if (p < g.npat)
-                        w[p] = *reinterpret_cast<const uint4*>(a16 + g.seg(blk, p) + static_cast<int64_t>(r0 + r) * 8);
-#pragma unroll
-                for (int p = 0; p < kDirectPatterns; p++) {
-                    if (p < g.npat) {
-                        const T* xg = xq + g.off[p];
-                        gather_word<T, true>(w[p].x, xg, xg, 0, acc);
-                        gather_word<T, true>(w[p].y, xg, xg, 0, acc);
-                        gather_word<T, true>(w[p].z, xg, xg, 0, acc);
-                        gather_word<T, true>(w[p].w, xg, xg, 0, acc);
-                    }
-                }
-            } else {
-                for (int p = 0; p < g.npat; p++) {
-                    const int ns = g.slots[p];
-                    gather_row<T>(a16 + g.seg(blk, p) + static_cast<int64_t>(r0 + r) * ns, ns, xq, xq + g.off[p], 0,
-                                  false, acc);
-                }
-            }
-            const int64_t row = g.block_row0(blk) + r0 + r;
-            double v = static_cast<double>(acc);
-            if (MODE == 1) v = static_cast<double>(y[row]) * -c + v;
-            if (MODE == 2) v = (b ? b[row] : 0.0) - v;
-            const Y yv = static_cast<Y>(v);
-            y[row] = yv;
-            mine.add(static_cast<double>(yv) * static_cast<double>(yv));
+        if (static_cast<int>(threadIdx.x) < nb) {
+            const int r = r0 + threadIdx.x;
+            const double v = static_cast<double>(row_sum<T, ALL8, false>(g, a16, blk, r, x + q * g.pcols, FastTable{}, nullptr));
+            const double yv = store_row<Y, MODE>(v, y, b, c, g.block_row0(blk) + r);
+            mine.add(yv * yv);
         }
         if (pu) {
             const Comp rs = block_sum_comp<kAxDirectRows>(mine, red);
@@ -2057,28 +2019,28 @@ cas_status fast_set_attributes()
 }
 cas_status fast_set_attributes_now()
 {
-    const int s32 = static_cast<int>(sizeof(float) * kTable32), s64 = static_cast<int>(sizeof(double) * kTable64);
+    const int tbl = kTableBytes;
     const int t32 = static_cast<int>(spmv_t_smem<float>(kMaxSc));
     const int t64 = static_cast<int>(spmv_t_smem<double>(1));
     const auto attr = cudaFuncAttributeMaxDynamicSharedMemorySize;
-    CAS_CUDA(cudaFuncSetAttribute(fast_spmv_kernel<float, float, 0, true>, attr, s32));
-    CAS_CUDA(cudaFuncSetAttribute(fast_spmv_kernel<float, float, 0, false>, attr, s32));
-    CAS_CUDA(cudaFuncSetAttribute(fast_spmv_kernel<float, float, 1, true>, attr, s32));
-    CAS_CUDA(cudaFuncSetAttribute(fast_spmv_kernel<float, float, 1, false>, attr, s32));
-    CAS_CUDA(cudaFuncSetAttribute(fast_spmv_kernel<float, float, 2, true>, attr, s32));
-    CAS_CUDA(cudaFuncSetAttribute(fast_spmv_kernel<float, float, 2, false>, attr, s32));
-    CAS_CUDA(cudaFuncSetAttribute(fast_spmv_kernel<double, double, 0, true>, attr, s64));
-    CAS_CUDA(cudaFuncSetAttribute(fast_spmv_kernel<double, double, 0, false>, attr, s64));
-    CAS_CUDA(cudaFuncSetAttribute(fast_spmv_kernel<double, double, 1, true>, attr, s64));
-    CAS_CUDA(cudaFuncSetAttribute(fast_spmv_kernel<double, double, 1, false>, attr, s64));
-    CAS_CUDA(cudaFuncSetAttribute(fast_spmv_kernel<double, double, 2, true>, attr, s64));
-    CAS_CUDA(cudaFuncSetAttribute(fast_spmv_kernel<double, double, 2, false>, attr, s64));
-    CAS_CUDA(cudaFuncSetAttribute(fast_spmv_kernel<double, float, 0, true>, attr, s64));
-    CAS_CUDA(cudaFuncSetAttribute(fast_spmv_kernel<double, float, 0, false>, attr, s64));
-    CAS_CUDA(cudaFuncSetAttribute(fast_spmv_kernel<double, float, 1, true>, attr, s64));
-    CAS_CUDA(cudaFuncSetAttribute(fast_spmv_kernel<double, float, 1, false>, attr, s64));
-    CAS_CUDA(cudaFuncSetAttribute(fast_spmv_kernel<double, float, 2, true>, attr, s64));
-    CAS_CUDA(cudaFuncSetAttribute(fast_spmv_kernel<double, float, 2, false>, attr, s64));
+    CAS_CUDA(cudaFuncSetAttribute(fast_spmv_table_kernel<float, float, 0, true>, attr, tbl));
+    CAS_CUDA(cudaFuncSetAttribute(fast_spmv_table_kernel<float, float, 0, false>, attr, tbl));
+    CAS_CUDA(cudaFuncSetAttribute(fast_spmv_table_kernel<float, float, 1, true>, attr, tbl));
+    CAS_CUDA(cudaFuncSetAttribute(fast_spmv_table_kernel<float, float, 1, false>, attr, tbl));
+    CAS_CUDA(cudaFuncSetAttribute(fast_spmv_table_kernel<float, float, 2, true>, attr, tbl));
+    CAS_CUDA(cudaFuncSetAttribute(fast_spmv_table_kernel<float, float, 2, false>, attr, tbl));
+    CAS_CUDA(cudaFuncSetAttribute(fast_spmv_table_kernel<double, double, 0, true>, attr, tbl));
+    CAS_CUDA(cudaFuncSetAttribute(fast_spmv_table_kernel<double, double, 0, false>, attr, tbl));
+    CAS_CUDA(cudaFuncSetAttribute(fast_spmv_table_kernel<double, double, 1, true>, attr, tbl));
+    CAS_CUDA(cudaFuncSetAttribute(fast_spmv_table_kernel<double, double, 1, false>, attr, tbl));
+    CAS_CUDA(cudaFuncSetAttribute(fast_spmv_table_kernel<double, double, 2, true>, attr, tbl));
+    CAS_CUDA(cudaFuncSetAttribute(fast_spmv_table_kernel<double, double, 2, false>, attr, tbl));
+    CAS_CUDA(cudaFuncSetAttribute(fast_spmv_table_kernel<double, float, 0, true>, attr, tbl));
+    CAS_CUDA(cudaFuncSetAttribute(fast_spmv_table_kernel<double, float, 0, false>, attr, tbl));
+    CAS_CUDA(cudaFuncSetAttribute(fast_spmv_table_kernel<double, float, 1, true>, attr, tbl));
+    CAS_CUDA(cudaFuncSetAttribute(fast_spmv_table_kernel<double, float, 1, false>, attr, tbl));
+    CAS_CUDA(cudaFuncSetAttribute(fast_spmv_table_kernel<double, float, 2, true>, attr, tbl));
+    CAS_CUDA(cudaFuncSetAttribute(fast_spmv_table_kernel<double, float, 2, false>, attr, tbl));
     CAS_CUDA(cudaFuncSetAttribute(fast_spmv_t_kernel<float>, attr, t32));
     CAS_CUDA(cudaFuncSetAttribute(fast_spmv_t_kernel<double>, attr, t64));
     return CAS_OK;
@@ -2198,6 +2160,26 @@ cas_status tune_transpose(FastLayout& f, const std::vector<int64_t>& entries, cu
     return build(best);
 }
 
+// The patterns whose slices of x the table kernel keeps in shared memory: by
+// entries a row per column, while they fit.
+FastTable table_plan(const FastGeometry& g, size_t elem)
+{
+    FastTable t;
+    std::vector<int> order(g.npat);
+    for (int p = 0; p < g.npat; p++) order[p] = p;
+    std::stable_sort(order.begin(), order.end(), [&](int a, int b) {
+        return static_cast<int64_t>(g.slots[a]) * g.space[b] > static_cast<int64_t>(g.slots[b]) * g.space[a];
+    });
+    for (int p = 0; p < kMaxFastPatterns; p++) t.base[p] = -1;
+    const int room = static_cast<int>(kTableBytes / elem);
+    for (int p : order)
+        if (t.elems + g.space[p] <= room) {
+            t.base[p] = t.elems;
+            t.elems += g.space[p];
+        }
+    return t;
+}
+
 }  // namespace
 
 bool fast_supported(const PatternSet& ps)
@@ -2270,6 +2252,8 @@ cas_status fast_build(const DevicePatterns& dp, const PatternSet& ps, const uint
         chunk += (g.space[p] + kChunkCols - 1) / kChunkCols;
     }
     g.nchunks = chunk;
+    f.tab32 = table_plan(g, sizeof(float));
+    f.tab64 = table_plan(g, sizeof(double));
     CAS_REQUIRE(g.total_elems() < 0xFFFFFFFFLL, CAS_ERR_INVALID_ARGUMENT,
                 "blocked layout: 2^32 or more entries (with block padding) are not supported");
     const int64_t elems = std::max<int64_t>(g.total_elems(), 8);
@@ -2367,49 +2351,44 @@ cas_status fast_diag(const FastLayout& f, uint64_t* diag, cudaStream_t s)
     return CAS_OK;
 }
 
-int fast_ax_splits(int64_t nblocks) { return unit_splits(nblocks, sm_count(), kAxSplitMax); }
+int fast_ax_parts(int64_t nblocks)
+{
+    return static_cast<int>(nblocks <= kAxDirectBlocks ? nblocks * kAxSplitMax : sm_count());
+}
 
 template <typename T, typename Y>
 cas_status fast_spmv(const FastLayout& f, const T* x, Y* y, const double* b, const double* coef, double* part,
                      int* done_flag, int mode, cudaStream_t s, int* n_parts, const int* pdone, const FastActive* act)
 {
-    const int split = act ? 1 : fast_ax_splits(f.g.nblocks);
-    const int64_t units = f.g.nblocks * (act ? kAxSplitMax : split);
-    const int ctas = static_cast<int>(std::max<int64_t>(1, std::min<int64_t>(units, sm_count())));
-    if (n_parts) *n_parts = static_cast<int>(units);  // one norm partial per (block, split)
-    if (f.g.nblocks == 0) return CAS_OK;
-    const size_t smem = sizeof(T) * (sizeof(T) == 4 ? kTable32 : kTable64);
-    const bool direct = act || split == kAxSplitMax;
-    const bool staged = act || split != kAxSplitMax;
-    auto launch = [&](auto kern) -> cas_status {
-        { kern<<<ctas, kAxThreads, smem, s>>>(f.g, f.a16, x, y, b, coef, part, done_flag, pdone, act, split, ctas); cas::count_launch(); }
-        CAS_CHECK_LAUNCH();
-        return CAS_OK;
-    };
+    const FastGeometry& g = f.g;
+    if (n_parts) *n_parts = fast_ax_parts(g.nblocks);
+    if (g.nblocks == 0) return CAS_OK;
     bool all8 = true;
-    for (int p = 0; p < f.g.npat; p++) all8 = all8 && f.g.slots[p] == 8;
-    if (direct) {
-        const unsigned dgrid = static_cast<unsigned>(
-            std::max<int64_t>(1, std::min<int64_t>(f.g.nblocks * kAxSplitMax, 4LL * sm_count())));
-        const bool d8 = all8 && f.g.npat <= kDirectPatterns;
-        auto kd = d8 ? (mode == 0 ? fast_spmv_direct_kernel<T, Y, 0, true>
-                                  : (mode == 1 ? fast_spmv_direct_kernel<T, Y, 1, true>
-                                               : fast_spmv_direct_kernel<T, Y, 2, true>))
-                     : (mode == 0 ? fast_spmv_direct_kernel<T, Y, 0, false>
-                                  : (mode == 1 ? fast_spmv_direct_kernel<T, Y, 1, false>
-                                               : fast_spmv_direct_kernel<T, Y, 2, false>));
-        { kd<<<dgrid, kAxDirectRows, 0, s>>>(f.g, f.a16, x, y, b, coef, part, done_flag, pdone, act, ctas); cas::count_launch(); }
+    for (int p = 0; p < g.npat; p++) all8 = all8 && g.slots[p] == 8;
+    if (act || g.nblocks <= kAxDirectBlocks) {
+        const unsigned grid = static_cast<unsigned>(std::min<int64_t>(g.nblocks * kAxSplitMax, 4LL * sm_count()));
+        auto kd = all8 ? (mode == 0 ? fast_spmv_direct_kernel<T, Y, 0, true>
+                                    : (mode == 1 ? fast_spmv_direct_kernel<T, Y, 1, true>
+                                                 : fast_spmv_direct_kernel<T, Y, 2, true>))
+                       : (mode == 0 ? fast_spmv_direct_kernel<T, Y, 0, false>
+                                    : (mode == 1 ? fast_spmv_direct_kernel<T, Y, 1, false>
+                                                 : fast_spmv_direct_kernel<T, Y, 2, false>));
+        { kd<<<grid, kAxDirectRows, 0, s>>>(g, f.a16, x, y, b, coef, part, done_flag, pdone, act); cas::count_launch(); }
         CAS_CHECK_LAUNCH();
     }
-    if (!staged) return CAS_OK;
-    if (all8) {
-        if (mode == 0) return launch(fast_spmv_kernel<T, Y, 0, true>);
-        if (mode == 1) return launch(fast_spmv_kernel<T, Y, 1, true>);
-        return launch(fast_spmv_kernel<T, Y, 2, true>);
+    if (g.nblocks > kAxDirectBlocks) {
+        const FastTable& tab = sizeof(T) == 4 ? f.tab32 : f.tab64;
+        auto kt = all8 ? (mode == 0 ? fast_spmv_table_kernel<T, Y, 0, true>
+                                    : (mode == 1 ? fast_spmv_table_kernel<T, Y, 1, true>
+                                                 : fast_spmv_table_kernel<T, Y, 2, true>))
+                       : (mode == 0 ? fast_spmv_table_kernel<T, Y, 0, false>
+                                    : (mode == 1 ? fast_spmv_table_kernel<T, Y, 1, false>
+                                                 : fast_spmv_table_kernel<T, Y, 2, false>));
+        { kt<<<sm_count(), kAxThreads, sizeof(T) * static_cast<size_t>(tab.elems), s>>>(
+            g, tab, f.a16, x, y, b, coef, part, done_flag, pdone, act); cas::count_launch(); }
+        CAS_CHECK_LAUNCH();
     }
-    if (mode == 0) return launch(fast_spmv_kernel<T, Y, 0, false>);
-    if (mode == 1) return launch(fast_spmv_kernel<T, Y, 1, false>);
-    return launch(fast_spmv_kernel<T, Y, 2, false>);
+    return CAS_OK;
 }
 
 template <typename T>

@@ -17,12 +17,12 @@
 // lane and row, so that a warp reads a round with 8 coalesced loads.
 // round_phys() maps an entry's position in the sorted order to its place.
 //
-// Both copies group a block's entries by pattern, so that a CTA touches one
-// pattern's columns at a time.  A x stages that
-// pattern's slice of x in shared memory and gathers from there; A'y stages
-// the block's slice of y in shared memory and reduces the column-sorted
-// entries of one column chunk into a shared-memory accumulator.  Local
-// columns must fit 16 bits (index space per pattern <= 65536).
+// Both copies group a block's entries by pattern.  A x gathers a row's
+// entries of x from a table of the patterns' slices (see FastTable) or
+// through the caches; A'y stages the block's slice of y in shared memory and
+// reduces the column-sorted entries of one column chunk into a shared-memory
+// accumulator.  Local columns must fit 16 bits (index space per pattern <=
+// 65536).
 #pragma once
 #include <cstdint>
 
@@ -35,19 +35,18 @@ constexpr int kRound = 1024;             // G32 entries of one A'y round (32 lan
 constexpr int kLaneRun = kRound / 32;    // consecutive entries a lane reduces per round
 constexpr int kFastThreads = 1024;       // threads of the A'y kernel
 constexpr int kAxThreads = 1024;         // threads of the A x kernel
-constexpr int kAxRows = kBlockRows / kAxThreads;  // rows per thread in A x
-constexpr int kAxAhead = 3;              // index loads in flight per thread in A x
 constexpr int kChunkCols = 8192;         // column chunk of the A'y accumulators
 constexpr int kSubCols = 1024;           // column sub-chunk: the finest split of an A'y item
 constexpr int kSubPerChunk = kChunkCols / kSubCols;
 constexpr int kEvalRedMax = 4096;        // CTAs of each reduction of an evaluator training step
-constexpr int kAxSplitMax = 32;          // most CTAs sharing one block's rows in A x
-constexpr int kAxDirectRows = kAxThreads / 2;  // rows of a unit that gathers x without staging (one thread a row)
-static_assert(kBlockRows / kAxSplitMax <= kAxDirectRows, "a block split kAxSplitMax ways must fit the direct path");
+constexpr int kAxSplitMax = 32;          // units of a block in the direct A x, and A x partials per block of a batch
+constexpr int kAxDirectRows = kBlockRows / kAxSplitMax;  // rows of such a unit, one a thread
+constexpr int kAxDirectBlocks = 48;      // most blocks that A x does without a table (see fast_spmv_table_kernel)
+constexpr int kAxTableSplit = kBlockRows / kAxThreads;   // units of a block in the table A x, one row a thread
+static_assert(kAxTableSplit < kAxSplitMax, "a table unit's partials share the layout of the direct units'");
 constexpr int kAtySplitMax = 16;         // most CTAs sharing one A'y item's columns
 constexpr int kMaxFastPatterns = 32;
-constexpr int kTable32 = 57344;          // x entries staged per pattern, FP32
-constexpr int kTable64 = 28672;          // x entries staged per pattern, FP64
+constexpr int kTableBytes = 140 * 1024;  // most shared memory of the A x table; the rest of the SM's 256 KB is L1
 
 constexpr int kMaxProblems = 64;         // independent fits in one batched layout
 
@@ -194,6 +193,12 @@ struct FastTranspose {
     void* meta = nullptr;          // one device block holding every array above except partial
 };
 
+// The patterns whose slices of x the A x kernel keeps in shared memory.
+struct FastTable {
+    int base[kMaxFastPatterns];  // first table element of the pattern's slice, -1: not in the table
+    int elems = 0;
+};
+
 // One measured A'y schedule of the build-time autotuner.
 struct FastTuneEntry {
     int per_sc;
@@ -207,6 +212,7 @@ constexpr int kMaxTune = 12;
 
 struct FastLayout {
     FastGeometry g;
+    FastTable tab32, tab64;
     FastTuneEntry tune[kMaxTune];      // candidates timed at build (empty: default schedule)
     int ntune = 0;
     int tune_cached = 0;               // schedule taken from the per-process cache
@@ -253,24 +259,22 @@ cas_status fast_build(const DevicePatterns& dp, const PatternSet& ps, const uint
 bool fast_supported(const PatternSet& ps);
 void fast_free(FastLayout& f);
 
-// y = A x on the blocked layout; also writes partials of ||y||^2, one per
-// (block, row split) (part may be null; *n_parts = their number).  mode 0:
-// y = A x; 1: y = A x - coef * y (coef read from *coef); 2: y = b - A x (b
-// may be null: y = -A x).  done_flag set: nothing runs; pdone[q] set: the
+// y = A x on the blocked layout; also writes compensated partials of
+// ||y||^2 (part may be null; *n_parts = their number, fast_ax_parts).  mode
+// 0: y = A x; 1: y = A x - coef * y (coef read from *coef); 2: y = b - A x
+// (b may be null: y = -A x).  done_flag set: nothing runs; pdone[q] set: the
 // rows of problem q are skipped (their partials are 0).
 //
-// Without act a block's rows are split over ax_splits(nblocks) CTAs and the
-// partials are laid out [block][split].  With act only the listed problems'
-// blocks run, split by a factor the kernel derives from the listed blocks,
-// and the partials are laid out [block][kAxSplitMax] (splits not used are 0):
-// problem q's partials are the 2 * kAxSplitMax * (pblk0[q+1] - pblk0[q])
-// doubles from part + 2 * kAxSplitMax * pblk0[q].
+// With act only the listed problems' blocks run, and the partials are laid
+// out [block][kAxSplitMax] (those not used are 0): problem q's are the
+// 2 * kAxSplitMax * (pblk0[q+1] - pblk0[q]) doubles from part + 2 *
+// kAxSplitMax * pblk0[q].
 template <typename T, typename Y>
 cas_status fast_spmv(const FastLayout& f, const T* x, Y* y, const double* b, const double* coef, double* part,
                      int* done_flag, int mode, cudaStream_t s, int* n_parts, const int* pdone = nullptr,
                      const FastActive* act = nullptr);
-// Row splits per block of A x without an active list.
-int fast_ax_splits(int64_t nblocks);
+// Norm partials of A x without an active list.
+int fast_ax_parts(int64_t nblocks);
 
 // Partials of A' y on the blocked layout (FP32: float partials, FP64:
 // double partials; a null y stands for a vector of ones); columns are
