@@ -129,10 +129,26 @@ __device__ void compact_active(const int* __restrict__ pdone, int nprob, ActiveL
     if (t == 0) al->n = base[1] + base[2];
 }
 
-__global__ void bcompact_kernel(const int* __restrict__ pdone, int nprob, ActiveList* al)
+// Where the A'y units of a list come from (FP32, FP64 work list) and the CTAs
+// they are laid out for.
+struct Plans {
+    FastPlanView v32, v64;
+    float ctas;
+};
+
+__device__ void plan_list(const Plans& pl, ActiveList* al)
+{
+    __syncthreads();  // the list as the CTA's threads wrote it
+    fast_plan_active(pl.v32, al, al->units[0], al->nunits, pl.ctas);
+    fast_plan_active(pl.v64, al, al->units[1], al->nunits + 1, pl.ctas);
+}
+
+__global__ void __launch_bounds__(kBRedThreads) bcompact_kernel(const int* __restrict__ pdone, int nprob,
+                                                                ActiveList* al, Plans pl)
 {
     __shared__ int base[3];
     compact_active(pdone, nprob, al, base);
+    plan_list(pl, al);
 }
 
 // Partial (s, c) of one CTA into part[2 * (q * G + rank)].
@@ -322,14 +338,14 @@ __global__ void __launch_bounds__(kBVecThreads) bupdate_kernel(FastCols fc, cons
 // step (skipall, set while no problem has one due; the count of due
 // problems reset), with use_cond the condition of the replacement step's
 // graph node and the count of such steps run (nbody), and the list of
-// problems still active for the next iteration.
+// problems still active for the next iteration with its A'y units.
 template <bool COMP>
 __global__ void __launch_bounds__(kBRedThreads) bbeta_kernel(const double* __restrict__ part_rz,
                                                              const double* __restrict__ part_rr, int G,
                                                              const ActiveList* al, BDev d, int replace,
                                                              const double* __restrict__ part_dev,
                                                              const int* __restrict__ qgate, int plan_refine,
-                                                             ActiveList* next, int use_cond,
+                                                             ActiveList* next, Plans pl, int use_cond,
                                                              cudaGraphConditionalHandle cond)
 {
     __shared__ double smem[64];
@@ -386,6 +402,8 @@ __global__ void __launch_bounds__(kBRedThreads) bbeta_kernel(const double* __res
     __syncthreads();
     if (!s_last) return;
     __threadfence();
+    const int listed = next->n;
+    __syncthreads();  // read before the list changes
     if (threadIdx.x == 0) {
         *d.fin = 0;
         if (plan_refine > 0) {
@@ -399,6 +417,8 @@ __global__ void __launch_bounds__(kBRedThreads) bbeta_kernel(const double* __res
         }
     }
     compact_active(d.pdone, d.nprob, next, base);
+    __syncthreads();
+    if (next->n != listed) plan_list(pl, next);  // the list only shrinks here
 }
 
 // p = z + beta p (and the gather copy).
@@ -454,6 +474,7 @@ struct BatchSolver {
     int* flags = nullptr;  // [B][kBFlags] then pdone[B], ndone, alldone, pskip[B], nneed, skipall, fin, nbody
     ActiveList* act = nullptr;  // problems not retired (rebuilt every iteration)
     ActiveList* all = nullptr;  // every problem
+    uint32_t* units = nullptr;  // the A'y units of both lists
     std::vector<double> h_scal;
     std::vector<int> h_flags;
     cudaGraphExec_t graph = nullptr;
@@ -482,6 +503,10 @@ struct BatchSolver {
     }
     int nflags() const { return B * kBFlags + B + 2 + B + 2 + 2; }
     int nbody_index() const { return nflags() - 1; }
+    Plans plans() const
+    {
+        return Plans{fast_plan_view<float>(*f), fast_plan_view<double>(*f), static_cast<float>(sm_count())};
+    }
     dim3 vgrid() const { return dim3(static_cast<unsigned>(G)); }
 
     ~BatchSolver()
@@ -494,7 +519,7 @@ struct BatchSolver {
         if (s2) cudaStreamDestroy(s2);
         for (void* ptr : {(void*)x, (void*)r, (void*)z, (void*)p, (void*)dinv, (void*)pg32, q, (void*)q64,
                           (void*)part_q, (void*)part_a, (void*)part_b, (void*)part_c, (void*)scal,
-                          (void*)flags, (void*)act, (void*)all})
+                          (void*)flags, (void*)act, (void*)all, (void*)units})
             dfree(ptr);
     }
 
@@ -509,7 +534,7 @@ struct BatchSolver {
         const BDev d = dev();
         int* whole = sel == Sel::All ? nullptr : (sel == Sel::Active ? d.alldone : d.skipall);
         const int* per = sel == Sel::All ? nullptr : (sel == Sel::Active ? d.pdone : d.pskip);
-        if (sel == Sel::Active) { bcompact_kernel<<<1, 64, 0, s>>>(d.pdone, B, act); cas::count_launch(); }
+        if (sel == Sel::Active) { bcompact_kernel<<<1, kBRedThreads, 0, s>>>(d.pdone, B, act, plans()); cas::count_launch(); }
         const ActiveList* al = sel == Sel::All ? all : act;
         CAS_TRY((fast_spmv<double, double>(*f, x, q64, b, nullptr, part_q, whole, 2, s, nullptr, per, al)));
         return fast_spmv_t_partials<double>(*f, q64, whole, s, per, al);
@@ -543,7 +568,7 @@ struct BatchSolver {
             { bresidual_kernel<COMP, double><<<vgrid(), kBVecThreads, 0, s>>>(fc, t64, r, z, p, nullptr, dinv, al,
                                                                          part_a, part_b, restart ? 1 : 0, d, pdev,
                                                                          qgate); cas::count_launch(); }
-        { bbeta_kernel<COMP><<<B, kBRedThreads, 0, s>>>(part_a, part_b, G, al, d, 1, pdev, qgate, 0, nullptr, 0, 0); cas::count_launch(); }
+        { bbeta_kernel<COMP><<<B, kBRedThreads, 0, s>>>(part_a, part_b, G, al, d, 1, pdev, qgate, 0, nullptr, plans(), 0, 0); cas::count_launch(); }
         if (pdev) {
             if (mixed)
                 { brestart_kernel<float><<<vgrid(), kBVecThreads, 0, s>>>(P, al, z, p, pg32, d); cas::count_launch(); }
@@ -572,7 +597,7 @@ struct BatchSolver {
                                                                                                         : f->t64.partial),
                                                                   x, r, z, p, dinv, act, part_q, part_a, part_b, d); cas::count_launch(); }
         { bbeta_kernel<COMP><<<B, kBRedThreads, 0, s>>>(part_a, part_b, G, act, d, 0, nullptr, d.pdone,
-                                                       mixed ? std::max(o.refine_every, 1) : 0, act, use_cond,
+                                                       mixed ? std::max(o.refine_every, 1) : 0, act, plans(), use_cond,
                                                        cond); cas::count_launch(); }
         if (mixed)
             { bdirection_kernel<float><<<vgrid(), kBVecThreads, 0, s>>>(P, act, z, p, pg32, d); cas::count_launch(); }
@@ -738,7 +763,11 @@ struct BatchSolver {
                 h.list[qq] = qq < B ? qq : 0;
                 h.pos[qq] = qq < B ? qq : -1;
             }
+            const int64_t room = fast_plan_room(*f);
+            CAS_CUDA(dmalloc(&units, sizeof(uint32_t) * 4 * room));
+            for (int k = 0; k < 2; k++) h.units[k] = units + k * room;
             CAS_CUDA(cudaMemcpy(all, &h, sizeof h, cudaMemcpyHostToDevice));
+            for (int k = 0; k < 2; k++) h.units[k] = units + (2 + k) * room;
             CAS_CUDA(cudaMemcpy(act, &h, sizeof h, cudaMemcpyHostToDevice));
         }
         CAS_CUDA(dmalloc(&scal, sizeof(double) * B * kBSlots));
@@ -754,6 +783,9 @@ struct BatchSolver {
             A->diag_int, C, o.jacobi ? 1 : 0, dinv); cas::count_launch(); }
         CAS_CHECK_LAUNCH();
         const BDev d = dev();
+        // the units of both lists (no problem is retired yet)
+        for (ActiveList* al : {all, act}) { bcompact_kernel<<<1, kBRedThreads, 0, s>>>(d.pdone, B, al, plans()); cas::count_launch(); }
+        CAS_CHECK_LAUNCH();
         // ||A'b||^2 per problem
         CAS_TRY(fast_spmv_t_partials<double>(*f, b, nullptr, s, nullptr));
         { bnorm_kernel<double><<<vgrid(), kBVecThreads, 0, s>>>(fast_cols<double>(*f), static_cast<const double*>(f->t64.partial),

@@ -629,17 +629,6 @@ __device__ __forceinline__ int active_slot(const int* pref, int n, int i)
     return lo;
 }
 
-// Splits of a work unit when `units` units of a product are to fill `ctas`
-// CTAs: as many as keep every split unit in one wave, at most cap.  A few
-// units' time is set by their chains of dependent loads, not by their
-// bytes, so one wave of larger units beats two of smaller ones.
-__host__ __device__ __forceinline__ int unit_splits(int64_t units, int64_t ctas, int cap)
-{
-    if (units <= 0) return 1;
-    const int64_t k = ctas / units;
-    return static_cast<int>(k < 1 ? 1 : (k > cap ? cap : k));
-}
-
 // The index words of one row of a pattern (slots 16-bit columns).  STREAM:
 // past L1, whose lines stay with x.
 template <bool STREAM>
@@ -920,15 +909,21 @@ struct TView {
     const int* item_b1;
     const int64_t* item_part;
     const int* sc_piece0;
-    const int* sc_width;
     const int* piece_pat;
     const int* piece_ch0;
     const int* piece_ch1;
     const int* piece_acc;
-    const int* sc_item0;  // [nprob * nsc + 1]: items of problem q are [sc_item0[q * nsc], sc_item0[(q + 1) * nsc])
+    const uint32_t* units;
+    int nunits;
     int nsc;
-    int per_sc;
-    int nitems;
+    int npieces;
+};
+
+// The units of a list of one item per (block, chunk): splits of each chunk
+// (0: the list has its own units).
+struct BlockUnits {
+    int per_block = 0;
+    uint8_t splits[kMaxChunks];
 };
 
 // Column-sorted entries are reduced lane by lane.  For one block of an item,
@@ -1065,16 +1060,16 @@ __device__ __forceinline__ T lane_entries(const uint4* __restrict__ src, int k0,
     return sum;
 }
 
-// Lane 0 of each warp asks L2 for the first round of the warp's stretch in
-// the block whose table is bp (issued a block ahead, before its barrier).
-__device__ __forceinline__ void prefetch_first_round(const uint32_t* __restrict__ g32, const BlockPieces& bp)
+// Lane w asks L2 for the first round of warp w's stretch in the block whose
+// table is bp.
+__device__ __forceinline__ void prefetch_first_rounds(const uint32_t* __restrict__ g32, const BlockPieces& bp)
 {
     constexpr int kWarps = kFastThreads / 32;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    if (lane != 0) return;
+    static_assert(kWarps == 32, "a lane per warp");
+    const int w = threadIdx.x & 31;
     const int nrounds = bp.round0[bp.n];
-    const int v = nrounds * warp / kWarps;
-    if (v >= nrounds * (warp + 1) / kWarps) return;  // no stretch
+    const int v = nrounds * w / kWarps;
+    if (v >= nrounds * (w + 1) / kWarps) return;  // no stretch
     int k = 0;
     while (bp.round0[k + 1] <= v) k++;
     const uint32_t rbase = ((bp.lo[k] / kRound) + static_cast<uint32_t>(v - bp.round0[k])) * kRound;
@@ -1088,7 +1083,7 @@ __device__ __forceinline__ void prefetch_first_round(const uint32_t* __restrict_
 // may restage ytile after the next barrier.
 template <typename T>
 __device__ __forceinline__ void reduce_block(const uint32_t* __restrict__ g32, const BlockPieces& bp,
-                                             const BlockPieces* next, const T* __restrict__ ytile,
+                                             const T* __restrict__ ytile,
                                              T* __restrict__ acc, WarpRec<T>* recs)
 {
     constexpr int kWarps = kFastThreads / 32;
@@ -1163,7 +1158,6 @@ __device__ __forceinline__ void reduce_block(const uint32_t* __restrict__ g32, c
         const bool ended = __ballot_sync(0xffffffffu, any && !single) != 0;  // every lane votes, every round
         w_end = w_end || ended;
     }
-    if (next) prefetch_first_round(g32, *next);  // while the other warps finish this block
     if (lane == 0) {
         WarpRec<T>& rec = recs[warp];
         rec.valid = vr0 < vr1;
@@ -1339,43 +1333,104 @@ __device__ __forceinline__ void reduce_stretch(const uint32_t* __restrict__ g32,
     }
 }
 
-// Accumulator columns [a0, a1) of piece pc that split `split` of `nsplit`
-// covers: its share of the piece's column sub-chunks.
-__device__ __forceinline__ void piece_share(const FastGeometry& g, const TView& tv, int pc, int split, int nsplit,
-                                            int& a0, int& a1)
+// A piece in shared memory (loaded once by each CTA).
+struct PieceMeta {
+    int pat;
+    int sub0;  // first column sub-chunk
+    int w;     // columns
+    int acc;   // accumulator offset of the first column
+};
+
+// First entry of column sub-chunk j (in the pattern's own count of the
+// layout) of a block, the group's end past the pattern's last.
+__device__ __forceinline__ uint32_t sub_entry(const FastGeometry& g, const uint32_t* __restrict__ sub_start, int p,
+                                              int j, int64_t blk)
 {
-    const int p = tv.piece_pat[pc];
-    const int cl0 = (tv.piece_ch0[pc] - g.chunk0[p]) * kChunkCols;
-    const int w = min(g.space[p], (tv.piece_ch1[pc] - g.chunk0[p]) * kChunkCols) - cl0;
-    const int ns = (w + kSubCols - 1) / kSubCols;
-    a0 = min(w, ns * split / nsplit * kSubCols);
-    a1 = min(w, ns * (split + 1) / nsplit * kSubCols);
+    const int end = (p + 1 < g.npat ? g.chunk0[p + 1] : g.nchunks) * kSubPerChunk;
+    return j < end ? sub_start[blk * (static_cast<int64_t>(g.nchunks) * kSubPerChunk) + j]
+                   : static_cast<uint32_t>(g.seg(blk, p) + g.seg_len(blk, p));
+}
+
+// The columns of every piece that split `split` of K covers, by one warp: the
+// item's sub-chunks in piece order are cut where the entries of block blk
+// pass s / K of the item's.  (Cut by column counts, the columns that hold
+// most entries stayed in one unit: 1,024 columns hold up to 77% of a
+// pattern's entries, 64 up to 15%.)
+__device__ __forceinline__ void unit_share(const FastGeometry& g, const PieceMeta* pm, int npc,
+                                           const uint32_t* __restrict__ sub_start, int64_t blk, int split, int K,
+                                           int2* share)
+{
+    const int lane = threadIdx.x & 31;
+    int w = 0, ns = 0;
+    if (lane < npc) w = pm[lane].w;
+    int ck[2] = {0, npc}, cc[2] = {0, 0};  // first and end cut: piece, column
+    if (K > 1) {
+        uint32_t start = 0, len = 0;
+        if (lane < npc) {
+            ns = (w + kSubCols - 1) / kSubCols;
+            start = sub_entry(g, sub_start, pm[lane].pat, pm[lane].sub0, blk);
+            len = sub_entry(g, sub_start, pm[lane].pat, pm[lane].sub0 + ns, blk) - start;
+        }
+        uint32_t incl = len;
+#pragma unroll
+        for (int d = 1; d < 32; d <<= 1) {
+            const uint32_t u = __shfl_up_sync(0xffffffffu, incl, d);
+            if (lane >= d) incl += u;
+        }
+        const uint32_t total = __shfl_sync(0xffffffffu, incl, 31);
+        // half a warp for each cut
+        const int e = lane >> 4, l = lane & 15;
+        const int sp = split + e;
+        const uint32_t tgt = sp < K ? static_cast<uint32_t>(static_cast<uint64_t>(total) * sp / K) : 0;
+        int k = 0;  // the piece where the entries pass the target
+        for (int t = 0; t < npc; t++) k += __shfl_sync(0xffffffffu, incl, t) <= tgt;
+        const bool inside = sp > 0 && sp < K && k < npc;
+        const int kk = min(k, npc - 1);
+        const uint32_t goal = __shfl_sync(0xffffffffu, start, kk) + (tgt - __shfl_sync(0xffffffffu, incl - len, kk));
+        const int p = pm[kk].pat, sub0 = pm[kk].sub0;
+        // first sub-chunk that starts at or after the goal
+        int lo = 0, hi = __shfl_sync(0xffffffffu, ns, kk);
+        if (!inside) hi = 0;
+        while (__any_sync(0xffffffffu, lo < hi)) {
+            const int step = (hi - lo + 15) / 16, j = lo + l * step;
+            const unsigned at = __ballot_sync(0xffffffffu, j >= hi || sub_entry(g, sub_start, p, sub0 + j, blk) >= goal) >>
+                                (16 * e) & 0xFFFFu;
+            const int f = at ? __ffs(at) - 1 : 16;
+            const int nlo = f == 0 ? lo : lo + (f - 1) * step + 1;
+            if (f < 16) hi = min(hi, lo + f * step);
+            lo = min(nlo, hi);
+        }
+        // a cut past the last entry is the end (no entries: the first split covers all)
+        const int cut = sp == 0 ? 0 : (inside ? k : npc), col = inside ? lo * kSubCols : 0;
+        ck[0] = __shfl_sync(0xffffffffu, cut, 0);
+        cc[0] = __shfl_sync(0xffffffffu, col, 0);
+        ck[1] = __shfl_sync(0xffffffffu, cut, 16);
+        cc[1] = __shfl_sync(0xffffffffu, col, 16);
+    }
+    if (lane < npc) {
+        const int a0 = lane < ck[0] ? w : (lane == ck[0] ? min(w, cc[0]) : 0);
+        const int a1 = lane < ck[1] ? w : (lane == ck[1] ? min(w, cc[1]) : 0);
+        share[lane] = make_int2(a0, a1);
+    }
+    __syncwarp();
 }
 
 // The table of one block's pieces (entry ranges of their shares, the
 // accumulator offsets, the virtual rounds), by one warp.
-__device__ __forceinline__ void fill_pieces(const FastGeometry& g, const TView& tv, const uint32_t* __restrict__ sub_start,
-                                            int pc0, int pc1, int split, int nsplit, int64_t blk, BlockPieces& bp)
+__device__ __forceinline__ void fill_pieces(const FastGeometry& g, const PieceMeta* pm, int npc,
+                                            const uint32_t* __restrict__ sub_start, const int2* share, int64_t blk,
+                                            BlockPieces& bp)
 {
     const int lane = threadIdx.x & 31;
-    const int nsub = g.nchunks * kSubPerChunk;
-    const int npc = pc1 - pc0;
     uint32_t lo = 0, hi = 0;
     int off = 0, nr = 0;
     if (lane < npc) {
-        const int pc = pc0 + lane;
-        int a0, a1;
-        piece_share(g, tv, pc, split, nsplit, a0, a1);
+        const PieceMeta m = pm[lane];
+        const int a0 = share[lane].x, a1 = share[lane].y;
         if (a0 < a1) {
-            const int p = tv.piece_pat[pc];
-            const int ch0 = tv.piece_ch0[pc];
-            const int pat_sub_end = (p + 1 < g.npat ? g.chunk0[p + 1] : g.nchunks) * kSubPerChunk;
-            const int j0 = ch0 * kSubPerChunk + a0 / kSubCols;
-            const int j1 = ch0 * kSubPerChunk + (a1 + kSubCols - 1) / kSubCols;
-            lo = sub_start[blk * nsub + j0];
-            hi = j1 < pat_sub_end ? sub_start[blk * nsub + j1]
-                                  : static_cast<uint32_t>(g.seg(blk, p) + g.seg_len(blk, p));
-            off = tv.piece_acc[pc] - (ch0 - g.chunk0[p]) * kChunkCols;
+            lo = sub_entry(g, sub_start, m.pat, m.sub0 + a0 / kSubCols, blk);
+            hi = sub_entry(g, sub_start, m.pat, m.sub0 + (a1 + kSubCols - 1) / kSubCols, blk);
+            off = m.acc - (m.sub0 * kSubCols - g.chunk0[m.pat] * kChunkCols);
             if (lo < hi) nr = static_cast<int>((hi - 1) / kRound - lo / kRound) + 1;
         }
     }
@@ -1395,117 +1450,154 @@ __device__ __forceinline__ void fill_pieces(const FastGeometry& g, const TView& 
         bp.round0[0] = 0;
         bp.n = npc;
     }
+    __syncwarp();
 }
 
-// One work unit: split `split` of `nsplit` of item `item`, i.e. the partial
-// column sums of its share of super-chunk item_sc[item]'s columns (a share
-// of every piece's column sub-chunks) over the blocks [item_b0, item_b1),
-// written to those columns of partial + item_part[item] -
-// item_part[item_base].  A column's entries of a block are one run of the
-// sorted group, so splitting at sub-chunk bounds splits no run.
+template <typename T>
+struct AtyShared {
+    // two record sets: the stretch reduction alternates them per piece, so
+    // that warp 0 may still combine one piece's records while the other
+    // warps start on the next piece
+    WarpRec<T> recs[2][kFastThreads / 32];
+    BlockPieces bp[2];  // this block's piece table and the next one's
+    PieceMeta pm[kMaxChunks];
+    int sc_piece0[kMaxChunks + 1];
+    // the unit: what its loop over blocks needs.  In shared memory, because
+    // the reductions need all 64 registers: with these held or spilled, the
+    // FP64 A'y of 610 blocks took 3,020 us, 2,570 so.
+    int64_t out;             // offset of its partials
+    const T* yb;             // y of its first block
+    int b0, nblk;
+    int left;                // rows of the problem from its first block on
+    int pc0, npc;            // its pieces
+    int2 share[kMaxPieces];  // columns of the unit in each piece
+    int unit;                // the CTA's next unit (persistent schedules)
+    uint32_t pack;           // the unit of a block list
+};
+
+// Stages y of `nb` rows into the tile by asynchronous copies, 16 bytes each
+// where the slice is aligned (a batch's problems start at any row); the caller
+// waits for them (stage_wait) before its barrier.
+template <typename T>
+__device__ __forceinline__ void stage_y(const T* __restrict__ yb, int nb, T* __restrict__ ytile)
+{
+    if (!yb) {  // no y: a vector of ones (the column counts A'1)
+        for (int i = threadIdx.x; i < nb; i += kFastThreads) ytile[i] = T(1);
+        return;
+    }
+    constexpr int kPer = 16 / sizeof(T);
+    constexpr unsigned kSize = sizeof(T);
+    const bool aligned = (reinterpret_cast<uintptr_t>(yb) & 15) == 0;
+    const int nvec = aligned ? nb / kPer : 0;
+    const unsigned dst = static_cast<unsigned>(__cvta_generic_to_shared(ytile));
+    for (int i = threadIdx.x; i < nvec; i += kFastThreads)
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + 16u * i), "l"(yb + kPer * i) : "memory");
+    for (int i = nvec * kPer + threadIdx.x; i < nb; i += kFastThreads)
+        asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"(dst + kSize * i), "l"(yb + i), "n"(kSize) : "memory");
+}
+
+__device__ __forceinline__ void stage_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+
+// One work unit: split `split` of K of item `item`, i.e. the partial column
+// sums of its share of super-chunk item_sc[item]'s columns (unit_share by the
+// item's first block) over the blocks [item_b0, item_b1), written to those
+// columns of partial + item_part[item] - item_part[item_base].  A column's
+// entries of a block are one run of the sorted group, so splitting at
+// sub-chunk bounds splits no run.
 // STRETCH: each (block, piece) range is reduced on its own by the stretch
 // reduction (the FP64 items); else the block's pieces share one round list.
+//
+// A unit of a small product is a chain of dependent loads, so the chain is
+// short: the item's fields at once, then the first block's y (asynchronous
+// copies) beside the unit's share and the table of the block's pieces, whose
+// fields the CTA has in shared memory.
 template <typename T, bool STRETCH>
 __device__ __forceinline__ void aty_item(const FastGeometry& g, const TView& tv, const uint32_t* __restrict__ g32,
                                          const uint32_t* __restrict__ sub_start, const T* __restrict__ y,
                                          T* __restrict__ partial, int item, int item_base, int64_t y_block0,
-                                         int split, int nsplit, T* __restrict__ acc, T* __restrict__ ytile,
-                                         WarpRec<T> (*recs)[kFastThreads / 32], BlockPieces* bp,
-                                         const int* __restrict__ pdone)
+                                         int split, int K, T* __restrict__ acc, T* __restrict__ ytile,
+                                         AtyShared<T>& sh, const int* __restrict__ pdone)
 {
-    if (pdone && pdone[g.prob_of_block(tv.item_b0[item])]) return;  // retired problem: partials unused
-    const int sc = tv.item_sc[item];
-    const int pc0 = tv.sc_piece0[sc], pc1 = tv.sc_piece0[sc + 1];
-    const int nsub = g.nchunks * kSubPerChunk;
-    bool any = false;
-    for (int pc = pc0; pc < pc1; pc++) {
-        int a0, a1;
-        piece_share(g, tv, pc, split, nsplit, a0, a1);
-        any = any || a0 < a1;
-        T* ap = acc + tv.piece_acc[pc];
-        for (int i = a0 + threadIdx.x; i < a1; i += kFastThreads) ap[i] = 0;
-    }
-    if (!any) return;  // more splits than sub-chunks: nothing here
     const int warp = threadIdx.x >> 5;
-    const int64_t b0 = tv.item_b0[item], b1 = tv.item_b1[item];
-    if (!STRETCH && warp == 0) fill_pieces(g, tv, sub_start, pc0, pc1, split, nsplit, b0, bp[0]);
-    for (int64_t blk = b0; blk < b1; blk++) {
-        const int nb = static_cast<int>(g.block_rows(blk));
-        const int i = static_cast<int>(blk - b0);
-        __syncthreads();
-        if (!STRETCH && i == 0) prefetch_first_round(g32, bp[0]);
-        const T* yb = y ? y + (g.block_row0(blk) - g.block_row0(y_block0)) : nullptr;
-        if (!yb) {  // no y: a vector of ones (the column counts A'1)
-            for (int i = threadIdx.x; i < nb; i += kFastThreads) ytile[i] = T(1);
-        } else if ((reinterpret_cast<uintptr_t>(yb) & 15) == 0) {
-            // 16-byte loads, kInFlight per thread issued before their stores
-            // (FP32: the whole tile in two rounds; FP64 keeps its registers)
-            constexpr int kPer = 16 / sizeof(T);
-            constexpr int kInFlight = sizeof(T) == 4 ? 2 : 1;
-            const int nvec = nb / kPer;
-            const uint4* srcv = reinterpret_cast<const uint4*>(yb);
-            uint4* dst = reinterpret_cast<uint4*>(ytile);
-            for (int i0 = threadIdx.x; i0 < nvec; i0 += kInFlight * kFastThreads) {
-                uint4 v[kInFlight];
-#pragma unroll
-                for (int kk = 0; kk < kInFlight; kk++)
-                    if (i0 + kk * kFastThreads < nvec) v[kk] = __ldg(srcv + i0 + kk * kFastThreads);
-#pragma unroll
-                for (int kk = 0; kk < kInFlight; kk++)
-                    if (i0 + kk * kFastThreads < nvec) dst[i0 + kk * kFastThreads] = v[kk];
+    {
+        const int sc = tv.item_sc[item];
+        const int b0 = tv.item_b0[item], b1 = tv.item_b1[item];
+        const int64_t out = tv.item_part[item] - tv.item_part[item_base];
+        const int q = g.prob_of_block(b0);  // items never span problems
+        if (pdone && pdone[q]) return;      // retired problem: partials unused
+        const int64_t row0 = g.prow0[q] + static_cast<int64_t>(b0 - g.pblk0[q]) * kBlockRows;
+        const int left = static_cast<int>(g.prow0[q + 1] - row0);
+        const T* yb = y ? y + (row0 - g.block_row0(y_block0)) : nullptr;
+        stage_y(yb, min(left, kBlockRows), ytile);
+        if (warp == 0) {
+            const int pc0 = sh.sc_piece0[sc], npc = sh.sc_piece0[sc + 1] - pc0;
+            if (threadIdx.x == 0) {
+                sh.out = out;
+                sh.yb = yb;
+                sh.b0 = b0;
+                sh.nblk = b1 - b0;
+                sh.left = left;
+                sh.pc0 = pc0;
+                sh.npc = npc;
             }
-            for (int i = nvec * kPer + threadIdx.x; i < nb; i += kFastThreads) ytile[i] = yb[i];
-        } else {
-            for (int i = threadIdx.x; i < nb; i += kFastThreads) ytile[i] = yb[i];
+            unit_share(g, sh.pm + pc0, npc, sub_start, b0, split, K, sh.share);
+            fill_pieces(g, sh.pm + pc0, npc, sub_start, sh.share, b0, sh.bp[0]);
+            if (!STRETCH) prefetch_first_rounds(g32, sh.bp[0]);
         }
-        if (y && blk + 1 < tv.item_b1[item])  // the next block's y slice into L2
-            prefetch_l2(y + (g.block_row0(blk + 1) - g.block_row0(y_block0)),
-                        static_cast<int64_t>(g.block_rows(blk + 1)) * static_cast<int64_t>(sizeof(T)));
-        if constexpr (STRETCH) {
-            __syncthreads();
-            int flip = 0;
-            for (int pc = pc0; pc < pc1; pc++) {
-                int a0, a1;
-                piece_share(g, tv, pc, split, nsplit, a0, a1);
-                if (a0 >= a1) continue;
-                const int p = tv.piece_pat[pc];
-                const int ch0 = tv.piece_ch0[pc];
-                const int pat_sub_end = (p + 1 < g.npat ? g.chunk0[p + 1] : g.nchunks) * kSubPerChunk;
-                const int j0 = ch0 * kSubPerChunk + a0 / kSubCols;
-                const int j1 = ch0 * kSubPerChunk + (a1 + kSubCols - 1) / kSubCols;
-                const uint32_t e_lo = sub_start[blk * nsub + j0];
-                const uint32_t e_hi = j1 < pat_sub_end ? sub_start[blk * nsub + j1]
-                                                       : static_cast<uint32_t>(g.seg(blk, p) + g.seg_len(blk, p));
-                T* accc = acc + tv.piece_acc[pc] - (ch0 - g.chunk0[p]) * kChunkCols;
-                reduce_stretch<T>(g32, e_lo, e_hi, ytile, accc, recs[flip]);
-                flip ^= 1;
-            }
-            continue;
-        }
-        if (warp == 0 && blk + 1 < b1)  // the next block's table, a block ahead
-            fill_pieces(g, tv, sub_start, pc0, pc1, split, nsplit, blk + 1, bp[(i + 1) & 1]);
-        __syncthreads();
-        reduce_block<T>(g32, bp[i & 1], blk + 1 < b1 ? &bp[(i + 1) & 1] : nullptr, ytile, acc, recs[0]);
     }
     __syncthreads();
-    T* out = partial + (tv.item_part[item] - tv.item_part[item_base]);
-    for (int pc = pc0; pc < pc1; pc++) {
-        int a0, a1;
-        piece_share(g, tv, pc, split, nsplit, a0, a1);
-        const int o = tv.piece_acc[pc];
-        for (int i = a0 + threadIdx.x; i < a1; i += kFastThreads) out[o + i] = acc[o + i];
+    for (int k = 0; k < sh.npc; k++) {
+        T* ap = acc + sh.pm[sh.pc0 + k].acc;
+        for (int i = sh.share[k].x + threadIdx.x; i < sh.share[k].y; i += kFastThreads) ap[i] = 0;
+    }
+    for (int i = 0; i < sh.nblk; i++) {
+        if (i > 0) {
+            __syncthreads();  // the tile is free
+            stage_y(sh.yb ? sh.yb + static_cast<int64_t>(i) * kBlockRows : nullptr,
+                    min(sh.left - i * kBlockRows, kBlockRows), ytile);
+        }
+        if (i + 1 < sh.nblk) {
+            if (sh.yb)  // the next block's y slice into L2
+                prefetch_l2(sh.yb + static_cast<int64_t>(i + 1) * kBlockRows,
+                            min(sh.left - (i + 1) * kBlockRows, kBlockRows) * static_cast<int64_t>(sizeof(T)));
+            if (warp == 0) {  // and its table, a block ahead
+                fill_pieces(g, sh.pm + sh.pc0, sh.npc, sub_start, sh.share, sh.b0 + i + 1, sh.bp[(i + 1) & 1]);
+                if (!STRETCH) prefetch_first_rounds(g32, sh.bp[(i + 1) & 1]);
+            }
+        }
+        stage_wait();
+        __syncthreads();
+        const BlockPieces& bp = sh.bp[i & 1];
+        if constexpr (STRETCH) {
+            int flip = 0;
+            for (int k = 0; k < bp.n; k++) {
+                const uint32_t lo = bp.lo[k], hi = bp.hi[k];
+                if (lo >= hi) continue;
+                reduce_stretch<T>(g32, lo, hi, ytile, acc + bp.acc_off[k], sh.recs[flip]);
+                flip ^= 1;
+            }
+        } else {
+            reduce_block<T>(g32, bp, ytile, acc, sh.recs[0]);
+        }
+    }
+    __syncthreads();
+    T* out = partial + sh.out;
+    for (int k = 0; k < sh.npc; k++) {
+        const int o = sh.pm[sh.pc0 + k].acc;
+        for (int i = sh.share[k].x + threadIdx.x; i < sh.share[k].y; i += kFastThreads) out[o + i] = acc[o + i];
     }
 }
 
-// A'y over a work list; a unit is one of the nsplit column splits of an
-// item.  With ctr (persistent schedule: one CTA per SM) the CTAs take units
-// in order from the counter ctr[0] until the list is done, so no SM idles
-// while units of uneven duration remain; which CTA runs a unit does not
-// change its output, so results stay bitwise reproducible.  The last CTA to
-// finish resets the counters for the next launch (launches on one work list
-// must therefore be stream-ordered).  Without ctr, CTA i runs unit i of the
-// items from item_base on.  With act (and ctr) the units are those of the
-// listed problems' items, split by a factor derived from their number.
+// A'y over a work list's units (unit_pack), or over those of the active
+// list's problems.  With ctr (persistent schedule: one CTA per SM) the CTAs
+// take units in order, the first by their index and the next from the counter
+// ctr[0], until the list is done, so no SM idles while units of uneven
+// duration remain; which CTA runs a unit does not change its output, so
+// results stay bitwise reproducible.  The last CTA to finish resets the
+// counters for the next launch (launches on one work list must therefore be
+// stream-ordered).  Without ctr, CTA i runs unit i.  bu.per_block set: the
+// units of a list of one item per (block, chunk), block by block from item
+// item_base on.
 template <typename T>
 __global__ void __launch_bounds__(kFastThreads, 1) fast_spmv_t_kernel(FastGeometry g, TView tv,
                                                                        const uint32_t* __restrict__ g32,
@@ -1515,46 +1607,55 @@ __global__ void __launch_bounds__(kFastThreads, 1) fast_spmv_t_kernel(FastGeomet
                                                                        const int* __restrict__ done, int item_base,
                                                                        int64_t y_block0, int* __restrict__ ctr,
                                                                        const int* __restrict__ pdone,
-                                                                       const FastActive* __restrict__ act, int nsplit)
+                                                                       const FastActive* __restrict__ act,
+                                                                       BlockUnits bu)
 {
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    // two record sets: the stretch reduction alternates them per piece, so
-    // that warp 0 may still combine one piece's records while the other
-    // warps start on the next piece
-    __shared__ WarpRec<T> recs[2][kFastThreads / 32];
-    __shared__ BlockPieces bp[2];  // this block's piece table and the next one's
+    __shared__ AtyShared<T> sh;
     constexpr bool kStretch = sizeof(T) == 8;  // FP64 items hold one chunk: few rounds per block
-    __shared__ int s_item;
-    __shared__ int pref[kMaxProblems + 1];
     if (done && *(volatile const int*)done) return;
     T* ytile = reinterpret_cast<T*>(smem_raw);  // first: its entries' byte offsets address it directly
     T* acc = ytile + kBlockRows;
+    for (int i = threadIdx.x; i < tv.npieces; i += kFastThreads) {
+        const int p = tv.piece_pat[i], c0 = tv.piece_ch0[i], c1 = tv.piece_ch1[i];
+        const int cl0 = (c0 - g.chunk0[p]) * kChunkCols;
+        sh.pm[i] = PieceMeta{p, c0 * kSubPerChunk, min(g.space[p], (c1 - g.chunk0[p]) * kChunkCols) - cl0, tv.piece_acc[i]};
+    }
+    for (int i = threadIdx.x; i <= tv.nsc; i += kFastThreads) sh.sc_piece0[i] = tv.sc_piece0[i];
     if (!ctr) {
         const int u = static_cast<int>(blockIdx.x);
-        aty_item<T, kStretch>(g, tv, g32, sub_start, y, partial, u / nsplit + item_base, item_base, y_block0,
-                              u % nsplit, nsplit, acc, ytile, recs, bp, pdone);
+        if (bu.per_block && threadIdx.x < 32) {
+            const int b = u / bu.per_block, r = u - b * bu.per_block, lane = threadIdx.x;
+            for (int c0 = 0, at = 0; c0 < g.nchunks; c0 += 32) {
+                const int K = c0 + lane < g.nchunks ? bu.splits[c0 + lane] : 0;
+                int incl = K;
+#pragma unroll
+                for (int d = 1; d < 32; d <<= 1) {
+                    const int v = __shfl_up_sync(0xffffffffu, incl, d);
+                    if (lane >= d) incl += v;
+                }
+                const int split = r - (at + incl - K);
+                if (split >= 0 && split < K) sh.pack = unit_pack(item_base + b * g.nchunks + c0 + lane, split, K);
+                at += __shfl_sync(0xffffffffu, incl, 31);
+            }
+        }
+        __syncthreads();
+        const uint32_t un = bu.per_block ? sh.pack : tv.units[u];
+        aty_item<T, kStretch>(g, tv, g32, sub_start, y, partial, static_cast<int>(un >> 8), item_base, y_block0,
+                              static_cast<int>(un >> 4 & 15u), static_cast<int>(un & 15u) + 1, acc, ytile, sh, pdone);
         return;
     }
-    int K = nsplit, units = tv.nitems * nsplit;
-    if (act) {
-        const int nit = active_prefix(act, pref, [&](int q) {
-            return tv.sc_item0[(q + 1) * tv.nsc] - tv.sc_item0[q * tv.nsc];
-        });
-        K = unit_splits(nit, gridDim.x, kAtySplitMax);
-        units = nit * K;
-    }
-    while (true) {
+    __syncthreads();
+    constexpr int kType = sizeof(T) == 4 ? 0 : 1;
+    const int units = act ? act->nunits[kType] : tv.nunits;
+    for (int u = static_cast<int>(blockIdx.x); u < units;) {
+        const uint32_t un = act ? act->units[kType][u] : tv.units[u];
+        aty_item<T, kStretch>(g, tv, g32, sub_start, y, partial, static_cast<int>(un >> 8), 0, 0,
+                              static_cast<int>(un >> 4 & 15u), static_cast<int>(un & 15u) + 1, acc, ytile, sh, pdone);
+        if (threadIdx.x == kFastThreads - 1) sh.unit = static_cast<int>(gridDim.x) + atomicAdd(ctr, 1);
         __syncthreads();
-        if (threadIdx.x == 0) s_item = atomicAdd(ctr, 1);
+        u = sh.unit;
         __syncthreads();
-        const int u = s_item;
-        if (u >= units) break;
-        int item = u / K;
-        if (act) {
-            const int slot = active_slot(pref, act->n, item);
-            item = tv.sc_item0[act->list[slot] * tv.nsc] + (item - pref[slot]);
-        }
-        aty_item<T, kStretch>(g, tv, g32, sub_start, y, partial, item, 0, 0, u % K, K, acc, ytile, recs, bp, pdone);
     }
     if (threadIdx.x == 0) {
         __threadfence();
@@ -1792,10 +1893,10 @@ void pack_pieces(const Pieces& pc, FastTranspose& t, MetaPack& mp)
 // Builds the work list of one A'y variant from the entry counts per (block,
 // chunk): super-chunks of at most per_sc chunks of columns, each split into
 // block ranges so that items carry about equal numbers of entries.
-// The most G32 entries of any item: its super-chunk's chunks over its blocks.
-int64_t max_item_entries(const FastGeometry& g, const std::vector<int64_t>& entries_bc, const Pieces& pc,
-                         const std::vector<int>& item_sc, const std::vector<int>& item_b0,
-                         const std::vector<int>& item_b1)
+// The G32 entries of every item: its super-chunk's chunks over its blocks.
+std::vector<int64_t> item_entries(const FastGeometry& g, const std::vector<int64_t>& entries_bc, const Pieces& pc,
+                                  const std::vector<int>& item_sc, const std::vector<int>& item_b0,
+                                  const std::vector<int>& item_b1)
 {
     const int nsc = pc.sc_width.empty() ? 0 : static_cast<int>(pc.sc_width.size());
     // prefix over blocks of every super-chunk's entries
@@ -1804,11 +1905,65 @@ int64_t max_item_entries(const FastGeometry& g, const std::vector<int64_t>& entr
         for (int sc = 0; sc < nsc; sc++) pre[(b + 1) * nsc + sc] = pre[b * nsc + sc];
         for (int ch = 0; ch < g.nchunks; ch++) pre[(b + 1) * nsc + pc.chunk_sc[ch]] += entries_bc[b * g.nchunks + ch];
     }
-    int64_t most = 0;
+    std::vector<int64_t> out(item_sc.size());
     for (size_t i = 0; i < item_sc.size(); i++)
-        most = std::max(most, pre[static_cast<size_t>(item_b1[i]) * nsc + item_sc[i]] -
-                                  pre[static_cast<size_t>(item_b0[i]) * nsc + item_sc[i]]);
-    return most;
+        out[i] = pre[static_cast<size_t>(item_b1[i]) * nsc + item_sc[i]] -
+                 pre[static_cast<size_t>(item_b0[i]) * nsc + item_sc[i]];
+    return out;
+}
+
+// The splits of every item (fixed cost and entries each) on the GPU: none
+// from kPlanWaves items a CTA on, else those of the best limit.
+std::vector<int> plan_splits(const std::vector<float>& fixed, const std::vector<float>& entries)
+{
+    const size_t n = fixed.size();
+    const float ctas = static_cast<float>(sm_count());
+    std::vector<int> K(n, 1);
+    if (n >= static_cast<size_t>(kPlanWaves) * sm_count()) return K;
+    float top = 0, best = 0, best_limit = 0;
+    for (size_t i = 0; i < n; i++) top = std::max(top, fixed[i] + entries[i]);
+    for (int j = 0; j < kPlanLimits; j++) {
+        const float limit = top * std::exp2(-0.25f * static_cast<float>(j));
+        float load = 0, longest = 0, units = 0;
+        for (size_t i = 0; i < n; i++) {
+            const int k = unit_split(fixed[i], entries[i], limit);
+            load += k * fixed[i] + entries[i];
+            longest = std::max(longest, fixed[i] + entries[i] / static_cast<float>(k));
+            units += static_cast<float>(k);
+        }
+        const float est = plan_estimate(units, load, longest, ctas);
+        if (j == 0 || est < best) {
+            best = est;
+            best_limit = limit;
+        }
+    }
+    for (size_t i = 0; i < n; i++) K[i] = unit_split(fixed[i], entries[i], best_limit);
+    return K;
+}
+
+// Units of a work list without an active list: in item order, and where
+// items are split, the most expensive first.
+void pack_units(const std::vector<int>& item_b0, const std::vector<int>& item_b1, const std::vector<int64_t>& entries,
+                bool fp64, FastTranspose& t, MetaPack& mp)
+{
+    const size_t n = entries.size();
+    std::vector<float> fixed(n), en(n);
+    for (size_t i = 0; i < n; i++) {
+        fixed[i] = unit_fixed(fp64, item_b1[i] - item_b0[i]);
+        en[i] = static_cast<float>(entries[i]);
+    }
+    const std::vector<int> K = plan_splits(fixed, en);
+    std::vector<int> order(n);
+    for (size_t i = 0; i < n; i++) order[i] = static_cast<int>(i);
+    if (n < static_cast<size_t>(kPlanWaves) * sm_count())
+        std::stable_sort(order.begin(), order.end(), [&](int a, int b) {
+            return fixed[a] + en[a] / static_cast<float>(K[a]) > fixed[b] + en[b] / static_cast<float>(K[b]);
+        });
+    std::vector<uint32_t> units;
+    for (int i : order)
+        for (int k = 0; k < K[i]; k++) units.push_back(unit_pack(i, k, K[i]));
+    t.nunits = static_cast<int>(units.size());
+    mp.add(units, &t.units);
 }
 
 cas_status build_items(const FastGeometry& g, const std::vector<int64_t>& entries_bc, int per_sc, int items_per_sm,
@@ -1870,7 +2025,9 @@ cas_status build_items(const FastGeometry& g, const std::vector<int64_t>& entrie
         }
         sc_item0.push_back(static_cast<int>(part_by_sc.size()));
         t.nitems = static_cast<int>(item_sc.size());
-        t.max_item_entries = max_item_entries(g, entries_bc, pc, item_sc, item_b0, item_b1);
+        const std::vector<int64_t> ie = item_entries(g, entries_bc, pc, item_sc, item_b0, item_b1);
+        t.max_item_entries = ie.empty() ? 0 : *std::max_element(ie.begin(), ie.end());
+        pack_units(item_b0, item_b1, ie, elem == sizeof(double), t, mp);
         mp.add(item_sc, &t.item_sc);
         mp.add(item_b0, &t.item_b0);
         mp.add(item_b1, &t.item_b1);
@@ -1908,7 +2065,18 @@ cas_status build_items(const FastGeometry& g, const std::vector<int64_t>& entrie
     }
     sc_item0.push_back(static_cast<int>(item_sc.size()));
     t.nitems = static_cast<int>(item_sc.size());
-    t.max_item_entries = max_item_entries(g, entries_bc, pc, item_sc, item_b0, item_b1);
+    const std::vector<int64_t> ie = item_entries(g, entries_bc, pc, item_sc, item_b0, item_b1);
+    t.max_item_entries = ie.empty() ? 0 : *std::max_element(ie.begin(), ie.end());
+    pack_units(item_b0, item_b1, ie, elem == sizeof(double), t, mp);
+    std::vector<float> grp_entries(static_cast<size_t>(g.nprob) * nsc, 0.0f);
+    std::vector<int> grp_blocks(grp_entries.size(), 0);
+    for (size_t grp = 0; grp < grp_entries.size(); grp++)
+        for (int i = sc_item0[grp]; i < sc_item0[grp + 1]; i++) {
+            grp_entries[grp] = std::max(grp_entries[grp], static_cast<float>(ie[i]));
+            grp_blocks[grp] = std::max(grp_blocks[grp], item_b1[i] - item_b0[i]);
+        }
+    mp.add(grp_entries, &t.grp_entries);
+    mp.add(grp_blocks, &t.grp_blocks);
     mp.add(item_sc, &t.item_sc);
     mp.add(item_b0, &t.item_b0);
     mp.add(item_b1, &t.item_b1);
@@ -1965,20 +2133,19 @@ cas_status build_block_items(const FastGeometry& g, FastTranspose& t)
 TView tview(const FastTranspose& t)
 {
     TView v;
-    v.per_sc = t.per_sc;
+    v.npieces = t.npieces;
     v.item_sc = t.item_sc;
     v.item_b0 = t.item_b0;
     v.item_b1 = t.item_b1;
     v.item_part = t.item_part;
     v.sc_piece0 = t.sc_piece0;
-    v.sc_width = t.sc_width;
     v.piece_pat = t.piece_pat;
     v.piece_ch0 = t.piece_ch0;
     v.piece_ch1 = t.piece_ch1;
     v.piece_acc = t.piece_acc;
-    v.sc_item0 = t.sc_item0;
+    v.units = t.units;
+    v.nunits = t.nunits;
     v.nsc = t.nsc;
-    v.nitems = t.nitems;
     return v;
 }
 
@@ -2307,6 +2474,11 @@ cas_status fast_build(const DevicePatterns& dp, const PatternSet& ps, const uint
         dfree(d_ce);
         for (size_t i = 0; i < ce.size(); i++) entries[i] = ce[i];
     }
+    for (int ch = 0; ch < g.nchunks; ch++) {
+        double sum = 0;
+        for (int64_t b = 0; b < g.nblocks; b++) sum += static_cast<double>(entries[b * g.nchunks + ch]);
+        f.chunk_entries[ch] = g.nblocks ? static_cast<float>(sum / static_cast<double>(g.nblocks)) : 0.0f;
+    }
     if (g.nblocks > 0) {
         CAS_TRY(tune_transpose(f, entries, s));
         // FP64 items hold one chunk, so the y slices would be read once per
@@ -2398,19 +2570,28 @@ cas_status fast_spmv_t_partials(const FastLayout& f, const T* y, int* done_flag,
     const FastTranspose& t = transpose_of<T>(f);
     if (t.nitems == 0) return CAS_OK;
     const size_t smem = spmv_t_smem<T>(t.per_sc);
-    // with an active list the kernel splits the units itself (persistent);
-    // else the items are split so that a short list still fills the GPU
-    const int nsplit = act ? 1 : unit_splits(t.nitems, sm_count(), kAtySplitMax);
-    const int units = t.nitems * nsplit;
     const bool persistent = t.persistent || act;
-    const unsigned grid = static_cast<unsigned>(persistent ? std::min(units, sm_count()) : units);
-    const unsigned pgrid = act ? static_cast<unsigned>(sm_count()) : grid;
-    int* ctr = persistent ? t.ctr : nullptr;
-    { fast_spmv_t_kernel<T><<<pgrid, kFastThreads, smem, s>>>(f.g, tview(t), f.g32, f.sub_start, y,
-                                                                  static_cast<T*>(t.partial), done_flag, 0, 0,
-                                                                  ctr, pdone, act, nsplit); cas::count_launch(); }
+    const unsigned grid = static_cast<unsigned>(
+        act ? sm_count() : (persistent ? std::min(t.nunits, sm_count()) : t.nunits));
+    { fast_spmv_t_kernel<T><<<grid, kFastThreads, smem, s>>>(f.g, tview(t), f.g32, f.sub_start, y,
+                                                             static_cast<T*>(t.partial), done_flag, 0, 0,
+                                                             persistent ? t.ctr : nullptr, pdone, act,
+                                                             BlockUnits{}); cas::count_launch(); }
     CAS_CHECK_LAUNCH();
     return CAS_OK;
+}
+
+template <typename T>
+FastPlanView fast_plan_view(const FastLayout& f)
+{
+    const FastTranspose& t = transpose_of<T>(f);
+    return FastPlanView{t.sc_item0, t.grp_entries, t.grp_blocks, t.nsc, sizeof(T) == 8};
+}
+
+int64_t fast_plan_room(const FastLayout& f)
+{
+    return std::max<int64_t>(std::max(f.t32.nitems, f.t64.nitems),
+                             static_cast<int64_t>(kPlanWaves) * sm_count() * kAtySplitMax);
 }
 
 template <typename T>
@@ -2499,11 +2680,22 @@ static cas_status eval_buffers(FastLayout& f, int64_t nb, cudaStream_t s)
 static cas_status eval_adjoint_partials(FastLayout& f, int64_t b0, int64_t b1, const float* g, cudaStream_t s)
 {
     const size_t smem = spmv_t_smem<float>(1);
-    const int items = static_cast<int>((b1 - b0) * f.g.nchunks);
-    { fast_spmv_t_kernel<float><<<items, kFastThreads, smem, s>>>(f.g, tview(f.tb), f.g32, f.sub_start, g,
-                                                                 f.eval_partial, nullptr,
-                                                                 static_cast<int>(b0 * f.g.nchunks), b0, nullptr,
-                                                                 nullptr, nullptr, 1); cas::count_launch(); }
+    // the chunks' splits from their mean entries in a block (a chunk of a
+    // block holds 1% to 100% of a pattern's)
+    const int nch = f.g.nchunks;
+    std::vector<float> fixed(static_cast<size_t>((b1 - b0) * nch), unit_fixed(false, 1)), entries(fixed.size());
+    for (size_t i = 0; i < entries.size(); i++) entries[i] = f.chunk_entries[i % nch];
+    const std::vector<int> K = plan_splits(fixed, entries);
+    BlockUnits bu;
+    for (int ch = 0; ch < nch; ch++) {
+        bu.splits[ch] = static_cast<uint8_t>(K[ch]);
+        bu.per_block += K[ch];
+    }
+    const int units = static_cast<int>(b1 - b0) * bu.per_block;
+    { fast_spmv_t_kernel<float><<<units, kFastThreads, smem, s>>>(f.g, tview(f.tb), f.g32, f.sub_start, g,
+                                                                  f.eval_partial, nullptr,
+                                                                  static_cast<int>(b0 * nch), b0, nullptr, nullptr,
+                                                                  nullptr, bu); cas::count_launch(); }
     CAS_CHECK_LAUNCH();
     return CAS_OK;
 }
@@ -2555,6 +2747,8 @@ template cas_status fast_spmv_t_partials<float>(const FastLayout&, const float*,
                                                 const FastActive*);
 template cas_status fast_spmv_t_partials<double>(const FastLayout&, const double*, int*, cudaStream_t, const int*,
                                                  const FastActive*);
+template FastPlanView fast_plan_view<float>(const FastLayout&);
+template FastPlanView fast_plan_view<double>(const FastLayout&);
 template FastCols fast_cols<float>(const FastLayout&);
 template FastCols fast_cols<double>(const FastLayout&);
 template cas_status fast_spmv_t<float>(const FastLayout&, const float*, float*, cudaStream_t);

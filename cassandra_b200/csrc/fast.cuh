@@ -36,7 +36,7 @@ constexpr int kLaneRun = kRound / 32;    // consecutive entries a lane reduces p
 constexpr int kFastThreads = 1024;       // threads of the A'y kernel
 constexpr int kAxThreads = 1024;         // threads of the A x kernel
 constexpr int kChunkCols = 8192;         // column chunk of the A'y accumulators
-constexpr int kSubCols = 1024;           // column sub-chunk: the finest split of an A'y item
+constexpr int kSubCols = 64;             // column sub-chunk: the finest split of an A'y item
 constexpr int kSubPerChunk = kChunkCols / kSubCols;
 constexpr int kEvalRedMax = 4096;        // CTAs of each reduction of an evaluator training step
 constexpr int kAxSplitMax = 32;          // units of a block in the direct A x, and A x partials per block of a batch
@@ -46,6 +46,7 @@ constexpr int kAxTableSplit = kBlockRows / kAxThreads;   // units of a block in 
 static_assert(kAxTableSplit < kAxSplitMax, "a table unit's partials share the layout of the direct units'");
 constexpr int kAtySplitMax = 16;         // most CTAs sharing one A'y item's columns
 constexpr int kMaxFastPatterns = 32;
+constexpr int kMaxChunks = kMaxFastPatterns * (65536 / kChunkCols);  // of a layout; pieces and super-chunks are no more
 constexpr int kTableBytes = 140 * 1024;  // most shared memory of the A x table; the rest of the SM's 256 KB is L1
 
 constexpr int kMaxProblems = 64;         // independent fits in one batched layout
@@ -149,12 +150,63 @@ static_assert(kRound == 1024 && kLaneRun == 32, "round_phys assumes 32 lanes x 3
 // order, rebuilt on the device before each iteration.  Given to the
 // products, it lets a few remaining small problems still fill the GPU: A x
 // and A'y split their work units (a block's rows, an item's columns) over
-// more CTAs the fewer units the listed problems have.
+// more CTAs the fewer units the listed problems have.  The A'y units of the
+// list are laid out when it changes (fast_plan_active).
 struct FastActive {
     int n;
     int list[kMaxProblems];
     int pos[kMaxProblems];  // slot of each problem in list, -1 if absent
+    int nunits[2];          // A'y units of the listed problems: FP32, FP64
+    uint32_t* units[2];     // (unit_pack), room for fast_plan_room() each
 };
+
+// A'y work units.  An item of a work list (a super-chunk's columns over a
+// block range) is one unit or is split by columns into up to kAtySplitMax.
+// What a unit takes is a fixed part (its fields, its share, its columns
+// cleared and written: 12,000 cycles), a part per block (y staged, the table,
+// barriers: 8,000) and its entries (280 cycles a round of 1,024 in FP32 and
+// 700 in FP64, which is the shared-memory bandwidth that y gathers and
+// accumulator updates at random banks leave), so it is counted in entries.  With fewer items than kPlanWaves a CTA, the items that cost more
+// than a limit are split; of kPlanLimits limits the one with the shortest
+// estimate is taken.  Items differ by a factor of 100 (the columns of an
+// edge or corner pattern that random play reaches, and those it does not), so
+// a few large ones set the time of a small product that does not split them.
+// A'y of the eight expanded patterns, us, FP32 / FP64, items whole or split by
+// column counts -> these units: 8 blocks 35 / 66 -> 29 / 49, 32 blocks
+// 68 / 199 -> 64 / 156, 64 blocks 126 / 335 -> 117 / 285; a training step's
+// 4 blocks 25 -> 17; a batch's iteration with 24 blocks left in three problems
+// 81 -> 59, with 15 left 43 -> 30.
+constexpr int kPlanWaves = 4;
+constexpr int kPlanLimits = 16;  // the most expensive item's cost, down in steps of 2^(1/4)
+
+// The fixed cost of a unit of `blocks` blocks, in entries.
+__host__ __device__ inline float unit_fixed(bool fp64, int blocks)
+{
+    return fp64 ? 18000.0f + 12000.0f * blocks : 40000.0f + 30000.0f * blocks;
+}
+
+__host__ __device__ inline uint32_t unit_pack(int item, int split, int K)
+{
+    return static_cast<uint32_t>(item) << 8 | static_cast<uint32_t>(split) << 4 | static_cast<uint32_t>(K - 1);
+}
+static_assert(kAtySplitMax == 16, "unit_pack: 4 bits for the split and its number");
+
+// Splits of an item of `entries` entries and fixed cost `fixed` that bring a
+// unit's cost to limit (at least two rounds a unit).
+__host__ __device__ inline int unit_split(float fixed, float entries, float limit)
+{
+    const float most = entries / (2.0f * kRound);
+    float k = limit > fixed ? ceilf(entries / (limit - fixed)) : static_cast<float>(kAtySplitMax);
+    k = k < most ? k : floorf(most);
+    return k < 1 ? 1 : (k > kAtySplitMax ? kAtySplitMax : static_cast<int>(k));
+}
+
+// What a schedule of `units` units takes on `ctas` CTAs: the longest unit in
+// one wave, else the mean load and a quarter of the longest.
+__host__ __device__ inline float plan_estimate(float units, float load, float longest, float ctas)
+{
+    return units <= ctas ? longest : (load / ctas > longest ? load / ctas : longest) + 0.25f * longest;
+}
 
 // Work list of one A'y variant.  Columns are grouped into "super-chunks":
 // sets of column pieces (whole 8192-column chunks of one pattern, or a
@@ -186,6 +238,10 @@ struct FastTranspose {
     int* item_b1 = nullptr;    // [nitems]
     int64_t* item_part = nullptr;  // [nitems] offset of the item's partials
     int* sc_item0 = nullptr;       // [nprob * nsc + 1] first entry of each (problem, super-chunk) in sc_part
+    uint32_t* units = nullptr;     // [nunits] the work units without an active list (unit_pack)
+    int nunits = 0;
+    float* grp_entries = nullptr;  // [nprob * nsc] most entries of an item of the (problem, super-chunk)
+    int* grp_blocks = nullptr;     // [nprob * nsc] most blocks of one
     int64_t* sc_part = nullptr;    // [nitems] partial offsets of the items, listed super-chunk by super-chunk
                                    // (block ranges in order): the order the column sums add them in
     void* partial = nullptr;       // float or double partials
@@ -218,6 +274,7 @@ struct FastLayout {
     int tune_cached = 0;               // schedule taken from the per-process cache
     uint16_t* a16 = nullptr;
     uint32_t* g32 = nullptr;
+    float chunk_entries[kMaxChunks];   // mean entries of each chunk in a block
     uint32_t* sub_start = nullptr;     // [nblocks][nchunks * kSubPerChunk] absolute index in G32 of the
                                        // first entry of every column sub-chunk (a chunk starts at its first)
     FastTranspose t32, t64;            // A'y work lists of the solvers (FP32, FP64)
@@ -235,6 +292,102 @@ struct FastLayout {
 struct EvalAdam {
     float lr, beta1, beta2, eps, l2, delta;
 };
+
+// Device view of a work list for fast_plan_active.
+struct FastPlanView {
+    const int* sc_item0;
+    const float* grp_entries;
+    const int* grp_blocks;
+    int nsc;
+    bool fp64;
+};
+template <typename T>
+FastPlanView fast_plan_view(const FastLayout& f);
+int64_t fast_plan_room(const FastLayout& f);  // units of either list at most
+
+// Lays out the units of the listed problems' items in units / *nunits; every
+// thread of one CTA calls (whole warps).  Items expensive under the chosen
+// limit come first.
+__device__ inline void fast_plan_active(const FastPlanView& pv, const FastActive* al, uint32_t* units, int* nunits,
+                                        float ctas)
+{
+    __shared__ float s_est[kPlanLimits], s_long[kPlanLimits], s_limit[kPlanLimits];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
+    const int ng = al->n * pv.nsc;
+    auto group = [&](int i, int& it0, int& nit, float& fixed, float& entries) {
+        const int grp = al->list[i / pv.nsc] * pv.nsc + i % pv.nsc;
+        it0 = pv.sc_item0[grp];
+        nit = pv.sc_item0[grp + 1] - it0;
+        fixed = unit_fixed(pv.fp64, pv.grp_blocks[grp]);
+        entries = pv.grp_entries[grp];
+    };
+    int it0, nit;
+    float fixed, entries;
+    float top = 0, items = 0;
+    for (int i = lane; i < ng; i += 32) {
+        group(i, it0, nit, fixed, entries);
+        if (nit > 0) top = fmaxf(top, fixed + entries);
+        items += nit;
+    }
+#pragma unroll
+    for (int d = 16; d > 0; d >>= 1) {
+        top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, d));
+        items += __shfl_xor_sync(0xffffffffu, items, d);
+    }
+    const int limits = items < kPlanWaves * ctas ? kPlanLimits : 1;  // the first limit splits nothing
+    for (int j = warp; j < limits; j += warps) {
+        const float limit = top * exp2f(-0.25f * j);
+        float load = 0, longest = 0, n = 0;
+        for (int i = lane; i < ng; i += 32) {
+            group(i, it0, nit, fixed, entries);
+            if (nit == 0) continue;
+            const int K = unit_split(fixed, entries, limit);
+            load += nit * (K * fixed + entries);
+            longest = fmaxf(longest, fixed + entries / K);
+            n += nit * K;
+        }
+#pragma unroll
+        for (int d = 16; d > 0; d >>= 1) {
+            load += __shfl_xor_sync(0xffffffffu, load, d);
+            n += __shfl_xor_sync(0xffffffffu, n, d);
+            longest = fmaxf(longest, __shfl_xor_sync(0xffffffffu, longest, d));
+        }
+        if (lane == 0) {
+            s_est[j] = plan_estimate(n, load, longest, ctas);
+            s_long[j] = longest;
+            s_limit[j] = limit;
+        }
+    }
+    __syncthreads();
+    if (warp == 0) {
+        int best = 0;
+        for (int j = 1; j < limits; j++)
+            if (s_est[j] < s_est[best]) best = j;
+        int at = 0;
+        for (int small = 0; small < 2; small++)
+            for (int i0 = 0; i0 < ng; i0 += 32) {
+                int K = 0;
+                nit = 0;
+                if (i0 + lane < ng) {
+                    group(i0 + lane, it0, nit, fixed, entries);
+                    K = unit_split(fixed, entries, s_limit[best]);
+                    if ((fixed + entries / K < 0.6f * s_long[best]) != (small != 0)) nit = 0;
+                }
+                int incl = nit * K;
+#pragma unroll
+                for (int d = 1; d < 32; d <<= 1) {
+                    const int u = __shfl_up_sync(0xffffffffu, incl, d);
+                    if (lane >= d) incl += u;
+                }
+                int o = at + incl - nit * K;
+                for (int it = 0; it < nit; it++)
+                    for (int k = 0; k < K; k++) units[o++] = unit_pack(it0 + it, k, K);
+                at += __shfl_sync(0xffffffffu, incl, 31);
+            }
+        if (lane == 0) *nunits = at;
+    }
+    __syncthreads();
+}
 
 // Device view used by the column reductions of the solver.
 struct FastCols {
