@@ -271,6 +271,114 @@ __global__ void __launch_bounds__(kBVecThreads) brestart_kernel(int64_t P, const
     }
 }
 
+// rz_new, rr (of k CTAs' partials) -> beta, relative residual, retirement of
+// problem q, by one CTA.  replace != 0: residual replacement (r.z replaced,
+// beta and the iteration count left alone).
+template <bool COMP, int THREADS>
+__device__ void beta_step(const double* part_rz, const double* part_rr, int G, int k, int q, const BDev& d, int replace,
+                          const double* part_dev, int plan_refine, double* smem)
+{
+    const int64_t o = 2 * static_cast<int64_t>(q) * G;
+    double* sc = d.scal + q * kBSlots;
+    int* fl = d.flags + q * kBFlags;
+    // the problem's state, loaded beside the partials
+    double rz = 0, bn2 = 0, tol = 0, ref = 0;
+    int iter = 0, iter_ref = 0;
+    if (threadIdx.x == 0) {
+        rz = sc[bRz];
+        bn2 = sc[bBn2];
+        tol = sc[bTol];
+        ref = sc[bRrRef];
+        iter = fl[bIter];
+        iter_ref = fl[bIterRef];
+    }
+    Comp a, b;
+    for (int i = threadIdx.x; i < k; i += THREADS) {
+        const double2 va = *reinterpret_cast<const double2*>(part_rz + o + 2 * i);
+        const double2 vb = *reinterpret_cast<const double2*>(part_rr + o + 2 * i);
+        a.add(Comp{va.x, va.y});
+        b.add(Comp{vb.x, vb.y});
+    }
+    block_sum_comp2<THREADS>(a, b, smem);
+    const double dev2 = part_dev ? bsum<COMP, THREADS>(part_dev + o, k, smem) : 0.0;
+    if (threadIdx.x == 0) {
+        const double rz_new = COMP ? a.value() : a.s, rr = COMP ? b.value() : b.s;
+        if (part_dev) fl[bRestart] = dev2 > kBRestartDeviation * kBRestartDeviation * rr ? 1 : 0;
+        const double res = bn2 > 0 ? sqrt(rr / bn2) : sqrt(rr);
+        if (!replace) {
+            sc[bBeta] = rz != 0 ? rz_new / rz : 0.0;
+            fl[bIter] = ++iter;
+        } else {
+            fl[bRefine] += 1;
+        }
+        sc[bRz] = rz_new;
+        sc[bRr] = rr;
+        sc[bRes] = res;
+        if (replace) {
+            sc[bRrRef] = rr;
+            fl[bIterRef] = iter;
+        }
+        const bool met = rr == 0 || (tol > 0 && res <= tol);
+        if (!isfinite(rz_new) || !isfinite(rr)) {
+            fl[bStatus] = CAS_ERR_BREAKDOWN;
+            retire(d, q);
+        } else if (!replace && plan_refine > 0) {
+            fl[bRestart] = 0;
+            const bool due = met || rr <= kBReplaceDrop * kBReplaceDrop * ref || iter - iter_ref >= plan_refine;
+            d.pskip[q] = due ? 0 : 1;
+            if (due) atomicAdd(d.nneed, 1);
+        } else if (met) {
+            retire(d, q);
+        }
+    }
+}
+
+// After the last problem's beta, by its CTA: the whole-launch gate of this
+// iteration's replacement step (skipall, set while no problem has one due;
+// the count of due problems reset), with use_cond the condition of the
+// replacement step's graph node and the count of such steps run (nbody), and
+// the list of problems still active for the next iteration with its A'y
+// units.
+__device__ void finish_step(const BDev& d, int plan_refine, ActiveList* next, const Plans& pl, int use_cond,
+                            cudaGraphConditionalHandle cond)
+{
+    __shared__ int base[3];
+    __shared__ int s_changed;
+    if (threadIdx.x == 0) {
+        const int listed = next->n, done = *(volatile int*)d.ndone, need = *(volatile int*)d.nneed;
+        s_changed = listed != d.nprob - done;  // the list only shrinks here
+        if (plan_refine > 0) {
+            const int skip = done == d.nprob || need == 0 ? 1 : 0;
+            *d.skipall = skip;
+            *d.nneed = 0;
+            if (use_cond) {
+                cudaGraphSetConditional(cond, skip ? 0u : 1u);
+                if (!skip) *d.nbody += 1;
+            }
+        }
+    }
+    __syncthreads();
+    if (!s_changed) return;
+    compact_active(d.pdone, d.nprob, next, base);
+    plan_list(pl, next);
+}
+
+// True in every thread of the last of n CTAs to call with this counter, which
+// that CTA resets; what the others wrote before is visible to it.
+__device__ bool last_to_arrive(int* counter, int n)
+{
+    __shared__ int s_last;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        __threadfence();
+        s_last = atomicAdd(counter, 1) == n - 1;
+        if (s_last) *counter = 0;
+        __threadfence();
+    }
+    __syncthreads();
+    return s_last != 0;
+}
+
 // alpha = rz / p'A'Ap per problem, then x += alpha p; r -= alpha A'A p;
 // z = D r; partials of r.z, r.r.  p'A'Ap is the sum of the A p norm
 // partials of the problem's blocks (kAxSplitMax per block), summed by every
@@ -279,8 +387,17 @@ __global__ void __launch_bounds__(kBVecThreads) brestart_kernel(int64_t P, const
 // space of A (a rank-deficient problem, or the residual at rounding level):
 // the problem retires and the FP64 true residual decides between converged
 // and a restart from it; a non-finite p'A'Ap is a breakdown.
+//
+// The step is latency: a chain of dependent loads (list, item tables,
+// partials) and of compensated adds.  So a CTA reads the chunks' partial
+// references once, a thread sums two columns at a time with their vector
+// elements loaded first, and the two norms are reduced together.  Eight
+// problems of 7 to 36 blocks, us with all, four, one left: 50, 24, 11.5 with
+// a column at a time, 39, 18, 9.3 so.  (With beta in the last CTA of a problem
+// instead of a launch: 52, 33, 20.5 for both, against 45, 24, 14.9: a fence
+// and an atomic for every CTA cost more than the launch.)
 template <bool COMP, typename T>
-__global__ void __launch_bounds__(kBVecThreads) bupdate_kernel(FastCols fc, const T* __restrict__ partial,
+__global__ void __launch_bounds__(kBVecThreads, 4) bupdate_kernel(FastCols fc, const T* __restrict__ partial,
                                                                double* __restrict__ x, double* __restrict__ r,
                                                                double* __restrict__ z, const double* __restrict__ p,
                                                                const double* __restrict__ dinv,
@@ -291,54 +408,78 @@ __global__ void __launch_bounds__(kBVecThreads) bupdate_kernel(FastCols fc, cons
 {
     __shared__ double smem[64];
     __shared__ double s_pap;
+    __shared__ int s_retired;  // read once: the first CTA may retire the problem meanwhile
+    __shared__ ChunkPartials ref[kMaxChunks];
     Slot sl;
-    if (!cta_slot(al, sl) || retired(d, sl.q)) return;
+    if (!cta_slot(al, sl)) return;
     const int q = sl.q;
+    if (threadIdx.x == 0) s_retired = retired(d, q);
+    fast_chunk_partials(fc, q, ref);
     const int b0 = fc.g.pblk0[q], nb = fc.g.pblk0[q + 1] - fc.g.pblk0[q];
     const double pap_sum = bsum<COMP, kBVecThreads>(part_q + 2 * static_cast<int64_t>(b0) * kAxSplitMax,
                                                     nb * kAxSplitMax, smem);
     if (threadIdx.x == 0) s_pap = pap_sum;
     __syncthreads();
-    const double pap = s_pap;
-    double* sc = d.scal + q * kBSlots;
-    const bool ok = pap > 0 && isfinite(pap);
-    if (sl.rank == 0 && threadIdx.x == 0) {
-        sc[bPap] = pap;
-        sc[bAlpha] = ok ? sc[bRz] / pap : 0.0;
-        if (!ok) {
-            if (!isfinite(pap)) d.flags[q * kBFlags + bStatus] = CAS_ERR_BREAKDOWN;
-            retire(d, q);
+    if (!s_retired) {
+        const double pap = s_pap;
+        double* sc = d.scal + q * kBSlots;
+        const bool ok = pap > 0 && isfinite(pap);
+        if (sl.rank == 0 && threadIdx.x == 0) {
+            sc[bPap] = pap;
+            sc[bAlpha] = ok ? sc[bRz] / pap : 0.0;
+            if (!ok) {
+                if (!isfinite(pap)) d.flags[q * kBFlags + bStatus] = CAS_ERR_BREAKDOWN;
+                retire(d, q);
+            }
+        }
+        if (ok) {
+            const double alpha = sc[bRz] / pap;
+            const int64_t P = fc.g.pcols, base = q * P;
+            const int64_t step = static_cast<int64_t>(sl.ranks) * blockDim.x;
+            constexpr int U = 2;
+            Comp rz, rr;
+            for (int64_t c0 = static_cast<int64_t>(sl.rank) * blockDim.x + threadIdx.x; c0 < P; c0 += U * step) {
+                int64_t c[U];
+                double xv[U], pv[U], rv[U], dv[U], sum[U];
+#pragma unroll
+                for (int u = 0; u < U; u++) {
+                    c[u] = c0 + u * step;
+                    const int64_t i = base + c[u];
+                    const bool in = c[u] < P;
+                    xv[u] = in ? x[i] : 0;
+                    pv[u] = in ? p[i] : 0;
+                    rv[u] = in ? r[i] : 0;
+                    dv[u] = in ? dinv[i] : 0;
+                }
+                fast_col_sums<T, U>(fc.g, ref, partial, c, sum);
+#pragma unroll
+                for (int u = 0; u < U; u++) {
+                    if (c[u] >= P) break;
+                    const int64_t i = base + c[u];
+                    x[i] = xv[u] + alpha * pv[u];
+                    const double rc = rv[u] - alpha * sum[u];
+                    const double zc = dv[u] * rc;
+                    r[i] = rc;
+                    z[i] = zc;
+                    bacc<COMP>(rz, rc * zc);
+                    bacc<COMP>(rr, rc * rc);
+                }
+            }
+            block_sum_comp2<kBVecThreads>(rz, rr, smem);
+            if (threadIdx.x == 0) {
+                const int64_t i = 2 * (static_cast<int64_t>(q) * gridDim.x + sl.rank);
+                part_rz[i] = rz.s;
+                part_rz[i + 1] = COMP ? rz.c : 0.0;
+                part_rr[i] = rr.s;
+                part_rr[i + 1] = COMP ? rr.c : 0.0;
+            }
         }
     }
-    if (!ok) return;
-    const double alpha = sc[bRz] / pap;
-    const int64_t P = fc.g.pcols, base = q * P;
-    Comp rz, rr;
-    for (int64_t c = static_cast<int64_t>(sl.rank) * blockDim.x + threadIdx.x; c < P;
-         c += static_cast<int64_t>(sl.ranks) * blockDim.x) {
-        const int64_t i = base + c;
-        const double s = fast_col_sum<T>(fc, partial, i);
-        x[i] += alpha * p[i];
-        const double rc = r[i] - alpha * s;
-        const double zc = dinv[i] * rc;
-        r[i] = rc;
-        z[i] = zc;
-        bacc<COMP>(rz, rc * zc);
-        bacc<COMP>(rr, rc * rc);
-    }
-    bwrite<COMP>(part_rz, sl, rz, smem);
-    bwrite<COMP>(part_rr, sl, rr, smem);
 }
 
-// rz_new, rr -> beta, relative residual, retirement.  replace != 0: residual
-// replacement (r.z replaced, beta and the iteration count left alone).
-//
-// With next (the step's beta kernel), the last CTA to finish also prepares
-// the next steps: the whole-launch gate of this iteration's replacement
-// step (skipall, set while no problem has one due; the count of due
-// problems reset), with use_cond the condition of the replacement step's
-// graph node and the count of such steps run (nbody), and the list of
-// problems still active for the next iteration with its A'y units.
+// beta of every problem, a CTA each (replace != 0: after a residual
+// replacement).  With next (the step's beta kernel), the last CTA to finish
+// prepares the next steps.
 template <bool COMP>
 __global__ void __launch_bounds__(kBRedThreads) bbeta_kernel(const double* __restrict__ part_rz,
                                                              const double* __restrict__ part_rr, int G,
@@ -349,76 +490,11 @@ __global__ void __launch_bounds__(kBRedThreads) bbeta_kernel(const double* __res
                                                              cudaGraphConditionalHandle cond)
 {
     __shared__ double smem[64];
-    __shared__ int s_last;
-    __shared__ int base[3];
     const int q = blockIdx.x;
     const int k = ranks_of(al, q, G);
-    if (!*(volatile const int*)(qgate + q) && k != 0) {
-        const int64_t o = 2 * static_cast<int64_t>(q) * G;
-        const double rz_new = bsum<COMP>(part_rz + o, k, smem);
-        const double rr = bsum<COMP>(part_rr + o, k, smem);
-        const double dev2 = part_dev ? bsum<COMP>(part_dev + o, k, smem) : 0.0;
-        if (threadIdx.x == 0) {
-            double* sc = d.scal + q * kBSlots;
-            int* fl = d.flags + q * kBFlags;
-            if (part_dev) fl[bRestart] = dev2 > kBRestartDeviation * kBRestartDeviation * rr ? 1 : 0;
-            const double rz = sc[bRz];
-            const double bn2 = sc[bBn2];
-            const double res = bn2 > 0 ? sqrt(rr / bn2) : sqrt(rr);
-            if (!replace) {
-                sc[bBeta] = rz != 0 ? rz_new / rz : 0.0;
-                fl[bIter] += 1;
-            } else {
-                fl[bRefine] += 1;
-            }
-            sc[bRz] = rz_new;
-            sc[bRr] = rr;
-            sc[bRes] = res;
-            if (replace) {
-                sc[bRrRef] = rr;
-                fl[bIterRef] = fl[bIter];
-            }
-            const bool met = rr == 0 || (sc[bTol] > 0 && res <= sc[bTol]);
-            if (!isfinite(rz_new) || !isfinite(rr)) {
-                fl[bStatus] = CAS_ERR_BREAKDOWN;
-                retire(d, q);
-            } else if (!replace && plan_refine > 0) {
-                fl[bRestart] = 0;
-                const bool due = met || rr <= kBReplaceDrop * kBReplaceDrop * sc[bRrRef] ||
-                                 fl[bIter] - fl[bIterRef] >= plan_refine;
-                d.pskip[q] = due ? 0 : 1;
-                if (due) atomicAdd(d.nneed, 1);
-            } else if (met) {
-                retire(d, q);
-            }
-        }
-    }
-    if (!next) return;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        __threadfence();  // this CTA's flags before its count
-        s_last = atomicAdd(d.fin, 1) == static_cast<int>(gridDim.x) - 1;
-    }
-    __syncthreads();
-    if (!s_last) return;
-    __threadfence();
-    const int listed = next->n;
-    __syncthreads();  // read before the list changes
-    if (threadIdx.x == 0) {
-        *d.fin = 0;
-        if (plan_refine > 0) {
-            const int skip = (*(volatile int*)d.alldone || atomicAdd(d.nneed, 0) == 0) ? 1 : 0;
-            *d.skipall = skip;
-            *d.nneed = 0;
-            if (use_cond) {
-                cudaGraphSetConditional(cond, skip ? 0u : 1u);
-                if (!skip) *d.nbody += 1;
-            }
-        }
-    }
-    compact_active(d.pdone, d.nprob, next, base);
-    __syncthreads();
-    if (next->n != listed) plan_list(pl, next);  // the list only shrinks here
+    if (!*(volatile const int*)(qgate + q) && k != 0)
+        beta_step<COMP, kBRedThreads>(part_rz, part_rr, G, k, q, d, replace, part_dev, plan_refine, smem);
+    if (next && last_to_arrive(d.fin, gridDim.x)) finish_step(d, plan_refine, next, pl, use_cond, cond);
 }
 
 // p = z + beta p (and the gather copy).

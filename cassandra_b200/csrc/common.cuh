@@ -170,4 +170,43 @@ __device__ inline Comp block_sum_comp(Comp v, double* smem)
     return r;
 }
 
+// Two compensated sums at once: their chains of dependent adds overlap.
+template <int BLOCK>
+__device__ inline void block_sum_comp2(Comp& a, Comp& b, double* smem)
+{
+    static_assert(BLOCK % 32 == 0 && BLOCK <= 512, "4 doubles a warp in 64");
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    auto tree = [](Comp& v, Comp& u) {
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            Comp w, x;
+            w.s = __shfl_down_sync(0xffffffffu, v.s, o);
+            w.c = __shfl_down_sync(0xffffffffu, v.c, o);
+            x.s = __shfl_down_sync(0xffffffffu, u.s, o);
+            x.c = __shfl_down_sync(0xffffffffu, u.c, o);
+            v.add(w);
+            u.add(x);
+        }
+    };
+    tree(a, b);
+    if (lane == 0) {
+        smem[4 * warp] = a.s;
+        smem[4 * warp + 1] = a.c;
+        smem[4 * warp + 2] = b.s;
+        smem[4 * warp + 3] = b.c;
+    }
+    __syncthreads();
+    a = b = Comp{};
+    if (warp == 0) {
+        if (lane < BLOCK / 32) {
+            a.s = smem[4 * lane];
+            a.c = smem[4 * lane + 1];
+            b.s = smem[4 * lane + 2];
+            b.c = smem[4 * lane + 3];
+        }
+        tree(a, b);
+    }
+    __syncthreads();
+}
+
 }  // namespace cas
