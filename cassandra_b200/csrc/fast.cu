@@ -129,52 +129,39 @@ constexpr uint32_t kNoPend = 0xFFFFFFFFu;
 constexpr int kSortPrefetchPieces = kSortTile * 4 / 4096;  // 4 KB pieces of a tile of 4-byte items
 
 struct SortSmem {
-    uint32_t hist[256];     // digit counts of the first pass (counted from the input)
-    uint32_t hist2[256];    // digit counts of the final pass (counted by the first pass's write-out)
-    uint32_t base[256];     // first output position of each digit
-    uint32_t running[256];  // entries of each digit written by earlier tiles
-    uint32_t tcount[256];   // the tile's entries of each digit
-    uint32_t tbase[256];    // the digit's first slot in the tile buffer
-    uint32_t pend_pos[256]; // final pass: the digit's last entry so far (kNoPend: none)
-    uint32_t pend_col[256]; //   and its column
-    uint32_t dst[256];      // output position of the tile buffer's slot 0 for the digit (mod 2^32)
-    uint32_t tend[256];     // end of the digit's slots in the tile buffer
-    uint32_t wcnt[kSortWarps][256];
+    uint32_t hist[256];   // digit counts of the first pass (counted from the input)
+    uint32_t hist2[256];  // digit counts of the final pass (counted by the first pass's write-out)
+    uint32_t dst[256];    // output position of the tile buffer's slot 0 for the digit (mod 2^32)
+    uint32_t wtot[kSortWarps];
+    uint16_t wcnt[kSortWarps][256];  // a warp's items of a digit, then their first slot in the tile buffer
     uint32_t buf[kSortTile];
 };
+static_assert(kSortThreads == 256, "one thread per digit");
 
-__device__ void block_exclusive_scan_256(const uint32_t* hist, uint32_t* out)
+// Exclusive scan over the CTA's threads of v.  Ends with a barrier behind the
+// reads of wtot's previous use only: the caller has one before the next.
+__device__ __forceinline__ uint32_t sort_scan(uint32_t v, uint32_t* wtot)
 {
-    // 256 values scanned by the first 8 warps; others idle.
-    __shared__ uint32_t warp_tot[8];
-    const int t = threadIdx.x;
-    uint32_t v = 0, incl = 0;
-    if (t < 256) {
-        v = hist[t];
-        incl = v;
-        const int lane = t & 31;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    uint32_t incl = v;
 #pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const uint32_t u = __shfl_up_sync(0xffffffffu, incl, o);
-            if (lane >= o) incl += u;
-        }
-        if (lane == 31) warp_tot[t >> 5] = incl;
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t u = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += u;
     }
+    if (lane == 31) wtot[warp] = incl;
     __syncthreads();
-    if (t < 256) {
-        uint32_t pre = 0;
-        for (int w = 0; w < (t >> 5); w++) pre += warp_tot[w];
-        out[t] = pre + incl - v;
-    }
-    __syncthreads();
+    uint32_t pre = 0;
+#pragma unroll
+    for (int w = 0; w < kSortWarps; w++) pre += w < warp ? wtot[w] : 0;
+    return pre + incl - v;
 }
 
-// The lanes of the warp whose valid 8-bit digit equals this lane's (from
-// eight ballots: no match instruction, which costs far more here).  Only
-// meaningful on valid lanes.
-__device__ __forceinline__ unsigned digit_peers(uint32_t d, bool valid)
+// The lanes of the warp whose 8-bit digit equals this lane's, from eight
+// ballots.
+__device__ __forceinline__ unsigned digit_peers(uint32_t d)
 {
-    unsigned peers = __ballot_sync(0xffffffffu, valid);
+    unsigned peers = 0xffffffffu;
 #pragma unroll
     for (int b = 0; b < 8; b++) {
         const bool bit = (d >> b) & 1u;
@@ -184,28 +171,124 @@ __device__ __forceinline__ unsigned digit_peers(uint32_t d, bool valid)
     return peers;
 }
 
-// One stable 8-bit counting-sort pass of a group's n items by the digit at
-// `shift`.  FROM_A16: the first pass, items made from the A16 segment
-// (local column << 16 | row << 2), written to out in sorted order while the
-// final pass's digit counts are gathered.  !FROM_A16: the final pass, items
-// read from `in`, written in G32's round order (round_phys of the sorted
-// position; out starts on a round boundary) with their end flags.
-template <bool FROM_A16>
-__device__ void sort_pass(const uint16_t* __restrict__ a16_in, const uint32_t* __restrict__ in, int n, int slots,
-                          int shift, uint32_t* __restrict__ out, SortSmem& sm)
+// What a thread keeps of its digit (thread t: digit t) over a pass's tiles.
+struct SortDigit {
+    uint32_t next;      // output position of the digit's next entry
+    uint32_t pend_pos;  // final pass: the digit's last entry so far (kNoPend: none)
+    uint32_t pend_col;  //   and its column
+};
+
+// One tile of a pass: count items (all kSortTile of them if WHOLE) from item
+// t0 of the group on.
+template <bool FROM_A16, bool WHOLE>
+__device__ __forceinline__ void sort_tile(const uint16_t* __restrict__ a16_in, const uint32_t* __restrict__ in, int t0,
+                                          int count, int slots_log2, uint32_t* __restrict__ out, SortDigit& dig,
+                                          SortSmem& sm)
 {
     constexpr bool FINAL = !FROM_A16;
+    constexpr int kShift = FROM_A16 ? 16 : 24;
     const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
     const unsigned lt_mask = (1u << lane) - 1;
-    auto item_at = [&](int e) -> uint32_t {
-        if (FROM_A16) return (static_cast<uint32_t>(a16_in[e]) << 16) | (static_cast<uint32_t>(e / slots) << 2);
-        return in[e];
-    };
+    uint16_t* mine = sm.wcnt[warp];
+    {
+        uint32_t* z = reinterpret_cast<uint32_t*>(mine);
+#pragma unroll
+        for (int i = 0; i < 128; i += 32) z[i + lane] = 0;
+    }
+    __syncwarp();
+    // 1. rank: the warp's items warp * 512 + 32 k + lane of the tile, in item
+    // order; items past the end take the last digit and rank behind it
+    const int i0 = warp * kSortWarpItems + lane;
+    uint32_t item[kSortPerThread];
+    uint16_t rk[kSortPerThread];  // rank among the warp's items of the same digit
+#pragma unroll
+    for (int k = 0; k < kSortPerThread; k++) {  // all loads first: one memory latency per tile
+        const int i = i0 + 32 * k;
+        item[k] = 0xFFFFFFFFu;
+        if (WHOLE || i < count)
+            item[k] = FROM_A16 ? static_cast<uint32_t>(a16_in[t0 + i]) << 16 |
+                                     static_cast<uint32_t>((t0 + i) >> slots_log2) << 2
+                               : in[t0 + i];
+    }
+#pragma unroll
+    for (int k = 0; k < kSortPerThread; k++) {
+        const uint32_t d = (item[k] >> kShift) & 255u;
+        const unsigned peers = digit_peers(d);
+        const uint32_t before = __popc(peers & lt_mask), c = mine[d];
+        __syncwarp();
+        if (before == 0) mine[d] = static_cast<uint16_t>(c + __popc(peers));
+        __syncwarp();
+        rk[k] = static_cast<uint16_t>(c + before);
+    }
+    __syncthreads();
+    // 2. digit t: the tile's entries, their first slot, each warp's first
+    uint32_t total = 0, cnt[kSortWarps];
+#pragma unroll
+    for (int w = 0; w < kSortWarps; w++) {
+        cnt[w] = total;
+        total += sm.wcnt[w][t];
+    }
+    const uint32_t start = sort_scan(total, sm.wtot);
+#pragma unroll
+    for (int w = 0; w < kSortWarps; w++) sm.wcnt[w][t] = static_cast<uint16_t>(start + cnt[w]);
+    sm.dst[t] = dig.next - start;
+    if (!WHOLE && t == 255) total -= kSortTile - count;
+    __syncthreads();
+    // 3. the tile into the buffer, digit by digit
+#pragma unroll
+    for (int k = 0; k < kSortPerThread; k++) sm.buf[mine[(item[k] >> kShift) & 255u] + rk[k]] = item[k];
+    __syncthreads();
+    // 4. out: consecutive buffer slots of a digit are consecutive positions
+#pragma unroll 4
+    for (int j = t; j < (WHOLE ? kSortTile : count); j += kSortThreads) {
+        uint32_t it = sm.buf[j];
+        const uint32_t pos = sm.dst[(it >> kShift) & 255u] + static_cast<uint32_t>(j);
+        if (FINAL) {
+            // an entry whose next one in the tile is of its digit ends its run
+            // if the columns differ; the digit's last one in the tile waits
+            const uint32_t nx = j + 1 < count ? sm.buf[j + 1] : ~it;
+            if ((nx >> 24) == (it >> 24) && (nx >> 16) != (it >> 16)) it |= 1u;
+            out[round_phys(pos)] = it;
+        } else {
+            out[pos] = it;
+            atomicAdd(&sm.hist2[it >> 24], 1u);
+        }
+    }
+    if (FINAL && total > 0) {
+        // the digit's entry waiting from an earlier tile ends its run unless
+        // this tile's first entry of the digit continues its column
+        const uint32_t first = sm.buf[start];
+        if (dig.pend_pos != kNoPend && (first >> 16) != dig.pend_col) out[round_phys(dig.pend_pos)] |= 1u;
+        dig.pend_pos = dig.next + total - 1;
+        dig.pend_col = sm.buf[start + total - 1] >> 16;
+    }
+    dig.next += total;
+    __syncthreads();
+}
+
+// One stable 8-bit counting-sort pass of a group's n items.  FROM_A16: the
+// first pass, by the low byte of the column, items made from the A16 segment
+// (local column << 16 | row << 2), written to out in sorted order while the
+// final pass's digit counts are gathered.  !FROM_A16: the final pass, by the
+// high byte, items read from `in`, written in G32's round order (round_phys of
+// the sorted position; out starts on a round boundary) with their end flags.
+//
+// Bound by instructions, the eight ballots of a ranked item first: whole tiles
+// run without bounds, a digit's counts and places stay with its thread, and
+// every lane reads its digit's count itself.  320M entries (5M rows of eight
+// expanded patterns): 4,230 us with bounds, divisions and a leader that hands
+// the count out, 3,240 us so.
+template <bool FROM_A16>
+__device__ __forceinline__ void sort_pass(const uint16_t* __restrict__ a16_in, const uint32_t* __restrict__ in, int n,
+                                          int slots, uint32_t* __restrict__ out, SortSmem& sm)
+{
+    constexpr bool FINAL = !FROM_A16;
+    const int t = threadIdx.x;
     if (FROM_A16) {
         // the digits (low column bytes) of the group, 8 columns per 16-byte
         // load (segments start on 1024-entry rounds), the last n % 8 one by
         // one
-        if (t < 256) sm.hist[t] = 0;
+        sm.hist[t] = 0;
         __syncthreads();
         const uint4* v = reinterpret_cast<const uint4*>(a16_in);
         for (int e = (n & ~7) + t; e < n; e += kSortThreads) atomicAdd(&sm.hist[a16_in[e] & 255u], 1u);
@@ -217,12 +300,10 @@ __device__ void sort_pass(const uint16_t* __restrict__ a16_in, const uint32_t* _
         }
         __syncthreads();
     }
-    block_exclusive_scan_256(FROM_A16 ? sm.hist : sm.hist2, sm.base);
-    if (t < 256) {
-        sm.running[t] = 0;
-        if (FROM_A16) sm.hist2[t] = 0;
-        sm.pend_pos[t] = kNoPend;
-    }
+    SortDigit dig{sort_scan(FROM_A16 ? sm.hist[t] : sm.hist2[t], sm.wtot), kNoPend, 0};
+    if (FROM_A16) sm.hist2[t] = 0;
+    __syncthreads();
+    const int slots_log2 = 31 - __clz(slots);  // 1, 2, 4 or 8
     for (int t0 = 0; t0 < n; t0 += kSortTile) {
         // the next tile's input into L2 while this one is ranked, in 4 KB
         // pieces rounded up to 16 bytes (inside the group's room: whole
@@ -239,88 +320,13 @@ __device__ void sort_pass(const uint16_t* __restrict__ a16_in, const uint32_t* _
                 asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(src + lo), "r"(len) : "memory");
             }
         }
-        // 1. rank: the warp's items t0 + warp * 512 + 32 k + lane, in item order
-        for (int i = lane; i < 256; i += 32) sm.wcnt[warp][i] = 0;
-        __syncwarp();
-        uint32_t item[kSortPerThread];
-        uint32_t rk[kSortPerThread];  // rank among the warp's items of the same digit
-#pragma unroll
-        for (int k = 0; k < kSortPerThread; k++) {  // all loads first: one memory latency per tile
-            const int e = t0 + warp * kSortWarpItems + k * 32 + lane;
-            item[k] = e < n ? item_at(e) : 0u;
-        }
-#pragma unroll
-        for (int k = 0; k < kSortPerThread; k++) {
-            const int e = t0 + warp * kSortWarpItems + k * 32 + lane;
-            const bool valid = e < n;
-            const uint32_t d = (item[k] >> shift) & 255u;
-            const unsigned peers = digit_peers(d, valid);
-            const int leader = __ffs(peers) - 1;
-            uint32_t before = 0;
-            if (valid && lane == leader) {
-                before = sm.wcnt[warp][d];
-                sm.wcnt[warp][d] = before + __popc(peers);
-            }
-            before = __shfl_sync(0xffffffffu, before, leader);
-            rk[k] = before + __popc(peers & lt_mask);
-            __syncwarp();
-        }
-        __syncthreads();
-        // 2. per digit: each warp's offset inside the tile's run of the digit
-        if (t < 256) {
-            uint32_t acc = 0;
-            for (int w = 0; w < kSortWarps; w++) {
-                const uint32_t c = sm.wcnt[w][t];
-                sm.wcnt[w][t] = acc;
-                acc += c;
-            }
-            sm.tcount[t] = acc;
-        }
-        __syncthreads();
-        block_exclusive_scan_256(sm.tcount, sm.tbase);
-        // 3. the tile into the buffer, digit by digit; per digit, the output
-        // position of buffer slot 0 and the end of its slots
-        if (t < 256) {
-            sm.dst[t] = sm.base[t] + sm.running[t] - sm.tbase[t];
-            sm.tend[t] = sm.tbase[t] + sm.tcount[t];
-        }
-#pragma unroll
-        for (int k = 0; k < kSortPerThread; k++) {
-            const int e = t0 + warp * kSortWarpItems + k * 32 + lane;
-            if (e < n) {
-                const uint32_t d = (item[k] >> shift) & 255u;
-                sm.buf[sm.tbase[d] + sm.wcnt[warp][d] + rk[k]] = item[k];
-            }
-        }
-        __syncthreads();
-        // 4. out: consecutive buffer slots of a digit are consecutive positions
-        const int tn = min(kSortTile, n - t0);
-        for (int j = t; j < tn; j += kSortThreads) {
-            uint32_t it = sm.buf[j];
-            const uint32_t d = (it >> shift) & 255u;
-            const uint32_t pos = sm.dst[d] + static_cast<uint32_t>(j);
-            if (FINAL) {
-                const bool last_in_tile = static_cast<uint32_t>(j) + 1 == sm.tend[d];
-                if (!last_in_tile && (sm.buf[j + 1] >> 16) != (it >> 16)) it |= 1u;
-                out[round_phys(pos)] = it;
-            } else {
-                out[pos] = it;
-                atomicAdd(&sm.hist2[it >> 24], 1u);
-            }
-        }
-        if (FINAL && t < 256 && sm.tcount[t] > 0) {
-            // the digit's entry waiting from an earlier tile ends its run
-            // unless this tile's first entry of the digit continues its column
-            const uint32_t first = sm.buf[sm.tbase[t]];
-            if (sm.pend_pos[t] != kNoPend && (first >> 16) != sm.pend_col[t]) out[round_phys(sm.pend_pos[t])] |= 1u;
-            sm.pend_pos[t] = sm.base[t] + sm.running[t] + sm.tcount[t] - 1;
-            sm.pend_col[t] = sm.buf[sm.tbase[t] + sm.tcount[t] - 1] >> 16;
-        }
-        __syncthreads();
-        if (t < 256) sm.running[t] += sm.tcount[t];
+        if (n - t0 >= kSortTile)
+            sort_tile<FROM_A16, true>(a16_in, in, t0, kSortTile, slots_log2, out, dig, sm);
+        else
+            sort_tile<FROM_A16, false>(a16_in, in, t0, n - t0, slots_log2, out, dig, sm);
     }
     // the last entry of every digit ends its run (the next has another digit)
-    if (FINAL && t < 256 && sm.pend_pos[t] != kNoPend) out[round_phys(sm.pend_pos[t])] |= 1u;
+    if (FINAL && dig.pend_pos != kNoPend) out[round_phys(dig.pend_pos)] |= 1u;
     __syncthreads();
 }
 
@@ -337,8 +343,8 @@ __global__ void __launch_bounds__(kSortThreads, kSortCtasPerSm) fast_sort_kernel
         const int p = static_cast<int>(grp - b * g.npat);
         const int n = static_cast<int>(g.seg_len(b, p));
         const int64_t seg = g.seg(b, p);
-        sort_pass<true>(a16 + seg, nullptr, n, g.slots[p], 16, mine, sm);
-        sort_pass<false>(nullptr, mine, n, g.slots[p], 24, g32 + seg, sm);
+        sort_pass<true>(a16 + seg, nullptr, n, g.slots[p], mine, sm);
+        sort_pass<false>(nullptr, mine, n, g.slots[p], g32 + seg, sm);
     }
 }
 
