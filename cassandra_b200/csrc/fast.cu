@@ -553,33 +553,6 @@ struct AccOf<double> {
     using type = double;
 };
 
-template <typename T>
-__device__ __forceinline__ void gather_row(const uint16_t* __restrict__ src, int ns, const T* __restrict__ table,
-                                           const T* __restrict__ xg, int cap, bool all_in_table,
-                                           typename AccOf<T>::type& acc)
-{
-    uint32_t w[4];
-    if (ns == 8) {
-        const uint4 u = *reinterpret_cast<const uint4*>(src);
-        w[0] = u.x, w[1] = u.y, w[2] = u.z, w[3] = u.w;
-    } else if (ns == 4) {
-        const uint2 u = *reinterpret_cast<const uint2*>(src);
-        w[0] = u.x, w[1] = u.y;
-    } else if (ns == 2) {
-        w[0] = *reinterpret_cast<const uint32_t*>(src);
-    } else {
-        w[0] = *src;
-    }
-#pragma unroll
-    for (int s = 0; s < 8; s++) {
-        if (s < ns) {
-            const uint32_t c = (w[s >> 1] >> ((s & 1) * 16)) & 0xFFFFu;
-            acc += static_cast<typename AccOf<T>::type>(all_in_table || static_cast<int>(c) < cap ? table[c]
-                                                                                               : __ldg(xg + c));
-        }
-    }
-}
-
 // Asks L2 to fetch [p, p + bytes) (the 16-byte words wholly inside it), in
 // 4 KB bulk prefetches spread over the CTA's threads.  A hint: the data is
 // read later with ordinary loads.
@@ -1674,23 +1647,27 @@ __global__ void __launch_bounds__(kFastThreads, 1) fast_spmv_t_kernel(FastGeomet
 }
 
 // Evaluator forward on a row range: score[r - row0] = sum_j w[col_rj], one
-// thread per row, 16-byte index loads, gathers of w through L1/L2 (the range
-// is a minibatch, too short to amortise staging w in shared memory).
-__global__ void __launch_bounds__(256) fast_rows_forward_kernel(FastGeometry g, const uint16_t* __restrict__ a16,
-                                                                const float* __restrict__ w, int64_t row0,
-                                                                int64_t row1, float* __restrict__ out)
+// thread per row (row_sum), gathers of w through L1/L2 (the range is a
+// minibatch, too short to amortise staging w in shared memory).
+constexpr int kEvalRows = 128;  // threads of a CTA
+
+template <bool ALL8>
+__device__ __forceinline__ float eval_row(const FastGeometry& g, const uint16_t* __restrict__ a16,
+                                          const float* __restrict__ w, int64_t r)
+{
+    int64_t b, rb;
+    g.locate_row(r, b, rb);
+    return row_sum<float, ALL8, false>(g, a16, b, static_cast<int>(rb), w + g.col_base(b), FastTable{}, nullptr);
+}
+
+template <bool ALL8>
+__global__ void __launch_bounds__(kEvalRows) fast_rows_forward_kernel(FastGeometry g, const uint16_t* __restrict__ a16,
+                                                                      const float* __restrict__ w, int64_t row0,
+                                                                      int64_t row1, float* __restrict__ out)
 {
     for (int64_t r = row0 + static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; r < row1;
-         r += static_cast<int64_t>(gridDim.x) * blockDim.x) {
-        int64_t b, rb;
-        g.locate_row(r, b, rb);
-        const float* wq = w + g.col_base(b);
-        float acc = 0;
-        for (int p = 0; p < g.npat; p++)
-            gather_row<float>(a16 + g.seg(b, p) + rb * g.slots[p], g.slots[p], wq + g.off[p], wq + g.off[p], 0, false,
-                              acc);
-        out[r - row0] = acc;
-    }
+         r += static_cast<int64_t>(gridDim.x) * blockDim.x)
+        out[r - row0] = eval_row<ALL8>(g, a16, w, r);
 }
 
 // Dense column sums of per-block partials laid out [block][cols].
@@ -1708,30 +1685,27 @@ __global__ void block_partial_sum_kernel(const float* __restrict__ partial, int 
 // Forward of a training step fused with its loss: per row the score (as in
 // fast_rows_forward_kernel), d = score - target, the Huber loss of d summed
 // per CTA into red[blockIdx.x] (FP64, deterministic tree), and the loss
-// gradient dscore = clamp(d, -delta, delta) / n for the adjoint.
-__global__ void __launch_bounds__(256) eval_loss_grad_kernel(FastGeometry g, const uint16_t* __restrict__ a16,
-                                                             const float* __restrict__ w,
-                                                             const float* __restrict__ target, int64_t row0,
-                                                             int64_t row1, float delta, float inv_n,
-                                                             float* __restrict__ dscore, double* __restrict__ red)
+// gradient dscore = clamp(d, -delta, delta) / n for the adjoint.  Bound by
+// latency: a row's index words are all loaded before its gathers (65,536 rows
+// of eight expanded patterns: 13.1 us pattern by pattern, 9.6 us so).
+template <bool ALL8>
+__global__ void __launch_bounds__(kEvalRows) eval_loss_grad_kernel(FastGeometry g, const uint16_t* __restrict__ a16,
+                                                                   const float* __restrict__ w,
+                                                                   const float* __restrict__ target, int64_t row0,
+                                                                   int64_t row1, float delta, float inv_n,
+                                                                   float* __restrict__ dscore, double* __restrict__ red)
 {
     __shared__ double smem[32];
     double hs = 0;
     for (int64_t r = row0 + static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; r < row1;
          r += static_cast<int64_t>(gridDim.x) * blockDim.x) {
-        int64_t b, rb;
-        g.locate_row(r, b, rb);
-        const float* wq = w + g.col_base(b);
-        float acc = 0;
-        for (int p = 0; p < g.npat; p++)
-            gather_row<float>(a16 + g.seg(b, p) + rb * g.slots[p], g.slots[p], wq + g.off[p], wq + g.off[p], 0, false,
-                              acc);
-        const float d = acc - target[r - row0];
+        const float tg = target[r - row0];
+        const float d = eval_row<ALL8>(g, a16, w, r) - tg;
         const float ad = fabsf(d);
         hs += ad < delta ? 0.5f * d * d : delta * (ad - 0.5f * delta);
         dscore[r - row0] = fminf(fmaxf(d, -delta), delta) * inv_n;
     }
-    const double t = block_sum<256>(hs, smem);
+    const double t = block_sum<kEvalRows>(hs, smem);
     if (threadIdx.x == 0) red[blockIdx.x] = t;
 }
 
@@ -1741,7 +1715,9 @@ __global__ void __launch_bounds__(256) eval_loss_grad_kernel(FastGeometry g, con
 // v = b2 v + (1 - b2) g^2, w -= lr / (1 - b1^t) * m / (sqrt(v) / sqrt(1 -
 // b2^t) + eps)).  ||w||^2 before the update is summed per CTA; the last CTA
 // (integer counter) adds the step's loss, sum(Huber)/n + l2 ||w||^2, to
-// *loss_sum, stores t and resets the counter.
+// *loss_sum, stores t and resets the counter.  The step's two powers are one
+// thread's work each, behind the loads of the first columns (166,212
+// columns, 4 blocks: 9.9 us with both in every thread, 8.5 us so).
 __global__ void __launch_bounds__(256) eval_adam_kernel(const float* __restrict__ partial, int nb, int64_t cols,
                                                         float* __restrict__ w, float* __restrict__ m,
                                                         float* __restrict__ v, int64_t* __restrict__ step,
@@ -1750,20 +1726,32 @@ __global__ void __launch_bounds__(256) eval_adam_kernel(const float* __restrict_
 {
     __shared__ double smem[32];
     __shared__ int last;
+    __shared__ float s_step, s_bc2;
     const int64_t t = *step + 1;  // read by every CTA before the last one stores t
-    const float step_size = static_cast<float>(o.lr / (1.0 - pow(static_cast<double>(o.beta1), static_cast<double>(t))));
-    const float bc2_sqrt = static_cast<float>(sqrt(1.0 - pow(static_cast<double>(o.beta2), static_cast<double>(t))));
+    if (threadIdx.x == 0)
+        s_step = static_cast<float>(o.lr / (1.0 - pow(static_cast<double>(o.beta1), static_cast<double>(t))));
+    if (threadIdx.x == 32)
+        s_bc2 = static_cast<float>(sqrt(1.0 - pow(static_cast<double>(o.beta2), static_cast<double>(t))));
     double wsq = 0;
-    for (int64_t c = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; c < cols;
-         c += static_cast<int64_t>(gridDim.x) * blockDim.x) {
-        float gc = 0;
-        for (int j = 0; j < nb; j++) gc += partial[static_cast<int64_t>(j) * cols + c];
-        const float wc = w[c];
+    bool powers = false;
+    const int64_t c0 = static_cast<int64_t>(blockIdx.x) * blockDim.x;
+    for (int64_t b = c0; b < cols; b += static_cast<int64_t>(gridDim.x) * blockDim.x) {
+        const int64_t c = b + threadIdx.x;
+        float gc = 0, wc = 0, mc = 0, vc = 0;
+        if (c < cols) {
+            for (int j = 0; j < nb; j++) gc += partial[static_cast<int64_t>(j) * cols + c];
+            wc = w[c];
+            mc = m[c];
+            vc = v[c];
+        }
+        if (!powers) __syncthreads();  // behind the first columns' loads
+        powers = true;
+        if (c >= cols) continue;
+        const float step_size = s_step, bc2_sqrt = s_bc2;
         wsq += static_cast<double>(wc) * wc;
         gc += (2.0f * o.l2) * wc;
-        float mc = m[c];
         mc += (1.0f - o.beta1) * (gc - mc);
-        const float vc = o.beta2 * v[c] + (1.0f - o.beta2) * gc * gc;
+        vc = o.beta2 * vc + (1.0f - o.beta2) * gc * gc;
         const float denom = sqrtf(vc) / bc2_sqrt + o.eps;
         w[c] = wc - step_size * (mc / denom);
         m[c] = mc;
@@ -2529,6 +2517,13 @@ cas_status fast_diag(const FastLayout& f, uint64_t* diag, cudaStream_t s)
     return CAS_OK;
 }
 
+static bool all_slots_8(const FastGeometry& g)
+{
+    bool all8 = true;
+    for (int p = 0; p < g.npat; p++) all8 = all8 && g.slots[p] == 8;
+    return all8;
+}
+
 int fast_ax_parts(int64_t nblocks)
 {
     return static_cast<int>(nblocks <= kAxDirectBlocks ? nblocks * kAxSplitMax : sm_count());
@@ -2541,8 +2536,7 @@ cas_status fast_spmv(const FastLayout& f, const T* x, Y* y, const double* b, con
     const FastGeometry& g = f.g;
     if (n_parts) *n_parts = fast_ax_parts(g.nblocks);
     if (g.nblocks == 0) return CAS_OK;
-    bool all8 = true;
-    for (int p = 0; p < g.npat; p++) all8 = all8 && g.slots[p] == 8;
+    const bool all8 = all_slots_8(g);
     if (act || g.nblocks <= kAxDirectBlocks) {
         const unsigned grid = static_cast<unsigned>(std::min<int64_t>(g.nblocks * kAxSplitMax, 4LL * sm_count()));
         auto kd = all8 ? (mode == 0 ? fast_spmv_direct_kernel<T, Y, 0, true>
@@ -2633,7 +2627,8 @@ cas_status fast_eval_forward(const FastLayout& f, int64_t row0, int64_t row1, co
                              cudaStream_t s)
 {
     if (row1 <= row0) return CAS_OK;
-    { fast_rows_forward_kernel<<<fgrid(row1 - row0, 256) * 4, 256, 0, s>>>(f.g, f.a16, w, row0, row1, score); cas::count_launch(); }
+    auto kernel = all_slots_8(f.g) ? fast_rows_forward_kernel<true> : fast_rows_forward_kernel<false>;
+    { kernel<<<fgrid(row1 - row0, kEvalRows) * 4, kEvalRows, 0, s>>>(f.g, f.a16, w, row0, row1, score); cas::count_launch(); }
     CAS_CHECK_LAUNCH();
     return CAS_OK;
 }
@@ -2729,12 +2724,13 @@ cas_status fast_eval_adam_step(FastLayout& f, int64_t row0, int64_t row1, const 
     const int64_t b0 = row0 / kBlockRows, b1 = (row1 + kBlockRows - 1) / kBlockRows;
     if (f.g.cols == 0 || n <= 0) return CAS_OK;
     CAS_TRY(eval_buffers(f, b1 - b0, s));
-    const unsigned g1 = std::min<unsigned>(fgrid(n, 256), kEvalRedMax);  // one thread per row up to 4 CTAs per SM
-    { eval_loss_grad_kernel<<<g1, 256, 0, s>>>(f.g, f.a16, w, target, row0, row1, o.delta, 1.0f / static_cast<float>(n),
-                                               f.eval_dscore, f.eval_red); cas::count_launch(); }
+    const unsigned g1 = std::min<unsigned>(fgrid(n, kEvalRows), kEvalRedMax);
+    auto loss = all_slots_8(f.g) ? eval_loss_grad_kernel<true> : eval_loss_grad_kernel<false>;
+    { loss<<<g1, kEvalRows, 0, s>>>(f.g, f.a16, w, target, row0, row1, o.delta, 1.0f / static_cast<float>(n),
+                                    f.eval_dscore, f.eval_red); cas::count_launch(); }
     CAS_CHECK_LAUNCH();
     CAS_TRY(eval_adjoint_partials(f, b0, b1, f.eval_dscore, s));
-    const unsigned g3 = std::min<unsigned>(fgrid(f.g.cols, 256), kEvalRedMax);
+    const unsigned g3 = static_cast<unsigned>(std::min<int64_t>((f.g.cols + 255) / 256, kEvalRedMax));  // a column a thread
     { eval_adam_kernel<<<g3, 256, 0, s>>>(f.eval_partial, static_cast<int>(b1 - b0), f.g.cols, w, m, v, step,
                                           loss_sum, f.eval_red, static_cast<int>(g1), f.eval_ctr, o,
                                           1.0 / static_cast<double>(n)); cas::count_launch(); }
