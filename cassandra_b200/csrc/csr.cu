@@ -430,22 +430,47 @@ __global__ void bound_check_kernel(const uint32_t* __restrict__ idx, int64_t n, 
 // Products.
 // ---------------------------------------------------------------------------
 
-// y = A x: one warp per row, lanes stride over the row's K indices (a
-// coalesced 4K-byte stream), gathers of x summed in FP64, warp-shuffle tree.
+// y = A x: a warp takes kSpmvRows rows at a time, its lanes stride over each
+// row's K indices (coalesced 4K-byte streams), gathers of x summed in FP64,
+// warp-shuffle trees.  Bound by the gathers' L1 lookups, one line a cycle and
+// SM (2M rows of 32 at random: 227 us), once the rows' chains of index, gather
+// and tree overlap: a row at a time 281 us (FP64 307), four 237 (261).  A part
+// of x in shared memory (64 to 180 KB, one CTA an SM) took 281 to 482.
+constexpr int kSpmvRows = 4;
+
 template <typename T>
 __global__ void __launch_bounds__(256) spmv_kernel(const uint32_t* __restrict__ idx, int64_t rows, int k,
                                                    const T* __restrict__ x, T* __restrict__ y)
 {
     const int lane = threadIdx.x & 31;
     const int64_t warps = static_cast<int64_t>(gridDim.x) * (blockDim.x >> 5);
-    for (int64_t r = static_cast<int64_t>(blockIdx.x) * (blockDim.x >> 5) + (threadIdx.x >> 5); r < rows;
-         r += warps) {
+    for (int64_t r = (static_cast<int64_t>(blockIdx.x) * (blockDim.x >> 5) + (threadIdx.x >> 5)) * kSpmvRows; r < rows;
+         r += warps * kSpmvRows) {
         const uint32_t* row = idx + r * k;
-        double acc = 0;
-        for (int j = lane; j < k; j += 32) acc += static_cast<double>(__ldg(x + __ldg(row + j)));
+        const int n = static_cast<int>(min(rows - r, static_cast<int64_t>(kSpmvRows)));
+        double acc[kSpmvRows] = {};
+        for (int j = lane; j < k; j += 32) {
+            uint32_t c[kSpmvRows];
+            T v[kSpmvRows];
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-        if (lane == 0) y[r] = static_cast<T>(acc);
+            for (int i = 0; i < kSpmvRows; i++)
+                if (i < n) c[i] = __ldg(row + static_cast<int64_t>(i) * k + j);
+#pragma unroll
+            for (int i = 0; i < kSpmvRows; i++)
+                if (i < n) v[i] = __ldg(x + c[i]);
+#pragma unroll
+            for (int i = 0; i < kSpmvRows; i++)
+                if (i < n) acc[i] += static_cast<double>(v[i]);
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+            for (int i = 0; i < kSpmvRows; i++) acc[i] += __shfl_xor_sync(0xffffffffu, acc[i], o);
+        double mine = acc[0];
+#pragma unroll
+        for (int i = 1; i < kSpmvRows; i++)
+            if (lane == i) mine = acc[i];
+        if (lane < n) y[r + lane] = static_cast<T>(mine);
     }
 }
 
@@ -500,7 +525,7 @@ template <typename T>
 cas_status spmv(const CsrView& a, const T* x, T* y, cudaStream_t s)
 {
     if (a.rows == 0) return CAS_OK;
-    { spmv_kernel<T><<<grid_for(a.rows, 8), 256, 0, s>>>(a.idx, a.rows, a.k, x, y); cas::count_launch(); }
+    { spmv_kernel<T><<<grid_for(a.rows, 8 * kSpmvRows), 256, 0, s>>>(a.idx, a.rows, a.k, x, y); cas::count_launch(); }
     CAS_CHECK_LAUNCH();
     return CAS_OK;
 }
