@@ -814,6 +814,8 @@ struct BatchSolver {
         b = d_b;
         mixed = o.precision == CAS_MIXED;
         G = 4 * sm_count();
+        CAS_REQUIRE(plans().v32.complete() && plans().v64.complete(), CAS_ERR_INVALID_ARGUMENT,
+                    "cas_solve_batched: the layout has no A'y plan");
         if (stream) {
             s = static_cast<cudaStream_t>(stream);
         } else {

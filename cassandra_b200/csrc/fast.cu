@@ -2062,15 +2062,17 @@ cas_status build_items(const FastGeometry& g, const std::vector<int64_t>& entrie
     const std::vector<int64_t> ie = item_entries(g, entries_bc, pc, item_sc, item_b0, item_b1);
     t.max_item_entries = ie.empty() ? 0 : *std::max_element(ie.begin(), ie.end());
     pack_units(item_b0, item_b1, ie, elem == sizeof(double), t, mp);
-    std::vector<float> grp_entries(static_cast<size_t>(g.nprob) * nsc, 0.0f);
-    std::vector<int> grp_blocks(grp_entries.size(), 0);
-    for (size_t grp = 0; grp < grp_entries.size(); grp++)
-        for (int i = sc_item0[grp]; i < sc_item0[grp + 1]; i++) {
-            grp_entries[grp] = std::max(grp_entries[grp], static_cast<float>(ie[i]));
-            grp_blocks[grp] = std::max(grp_blocks[grp], item_b1[i] - item_b0[i]);
-        }
-    mp.add(grp_entries, &t.grp_entries);
-    mp.add(grp_blocks, &t.grp_blocks);
+    if (g.nprob > 1) {
+        std::vector<float> grp_entries(static_cast<size_t>(g.nprob) * nsc, 0.0f);
+        std::vector<int> grp_blocks(grp_entries.size(), 0);
+        for (size_t grp = 0; grp < grp_entries.size(); grp++)
+            for (int i = sc_item0[grp]; i < sc_item0[grp + 1]; i++) {
+                grp_entries[grp] = std::max(grp_entries[grp], static_cast<float>(ie[i]));
+                grp_blocks[grp] = std::max(grp_blocks[grp], item_b1[i] - item_b0[i]);
+            }
+        mp.add(grp_entries, &t.grp_entries);
+        mp.add(grp_blocks, &t.grp_blocks);
+    }
     mp.add(item_sc, &t.item_sc);
     mp.add(item_b0, &t.item_b0);
     mp.add(item_b1, &t.item_b1);
@@ -2585,7 +2587,9 @@ template <typename T>
 FastPlanView fast_plan_view(const FastLayout& f)
 {
     const FastTranspose& t = transpose_of<T>(f);
-    return FastPlanView{t.sc_item0, t.grp_entries, t.grp_blocks, t.nsc, sizeof(T) == 8};
+    const bool one = f.g.nprob == 1;
+    return FastPlanView{one ? t.units : nullptr, one ? t.nunits : 0, t.sc_item0, t.grp_entries, t.grp_blocks, t.nsc,
+                        sizeof(T) == 8};
 }
 
 int64_t fast_plan_room(const FastLayout& f)

@@ -240,8 +240,9 @@ struct FastTranspose {
     int* sc_item0 = nullptr;       // [nprob * nsc + 1] first entry of each (problem, super-chunk) in sc_part
     uint32_t* units = nullptr;     // [nunits] the work units without an active list (unit_pack)
     int nunits = 0;
-    float* grp_entries = nullptr;  // [nprob * nsc] most entries of an item of the (problem, super-chunk)
-    int* grp_blocks = nullptr;     // [nprob * nsc] most blocks of one
+    float* grp_entries = nullptr;  // [nprob * nsc] most entries of an item of the (problem, super-chunk); null for
+                                   // one problem, whose active list takes `units`
+    int* grp_blocks = nullptr;     // [nprob * nsc] most blocks of one, likewise
     int64_t* sc_part = nullptr;    // [nitems] partial offsets of the items, listed super-chunk by super-chunk
                                    // (block ranges in order): the order the column sums add them in
     void* partial = nullptr;       // float or double partials
@@ -293,13 +294,21 @@ struct EvalAdam {
     float lr, beta1, beta2, eps, l2, delta;
 };
 
-// Device view of a work list for fast_plan_active.
+// Device view of a work list for fast_plan_active.  One problem is listed or
+// not, so its plan is the one made at build (units); several problems' units
+// are laid out from the costs of their (problem, super-chunk) groups, whose
+// items sc_item0 numbers (in a list of one problem sc_item0 counts sc_part's
+// entries, which are not the items when those run range by range).
 struct FastPlanView {
+    const uint32_t* units;
+    int nunits;
     const int* sc_item0;
     const float* grp_entries;
     const int* grp_blocks;
     int nsc;
     bool fp64;
+    // every array that fast_plan_active reads is there
+    bool complete() const { return nsc == 0 || units || (sc_item0 && grp_entries && grp_blocks); }
 };
 template <typename T>
 FastPlanView fast_plan_view(const FastLayout& f);
@@ -311,6 +320,13 @@ int64_t fast_plan_room(const FastLayout& f);  // units of either list at most
 __device__ inline void fast_plan_active(const FastPlanView& pv, const FastActive* al, uint32_t* units, int* nunits,
                                         float ctas)
 {
+    if (pv.units) {
+        const int n = al->n > 0 ? pv.nunits : 0;
+        for (int i = threadIdx.x; i < n; i += blockDim.x) units[i] = pv.units[i];
+        if (threadIdx.x == 0) *nunits = n;
+        __syncthreads();
+        return;
+    }
     __shared__ float s_est[kPlanLimits], s_long[kPlanLimits], s_limit[kPlanLimits];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
     const int ng = al->n * pv.nsc;
