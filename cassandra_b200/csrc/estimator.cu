@@ -112,6 +112,14 @@ __global__ void expand_kernel(const Slot* __restrict__ slots, const int64_t* __r
 constexpr int kEvalGroup = 16;   // slots per buffer pass (two tiles)
 constexpr int kEvalStride = 36;  // buffer words per slot: a quad's lanes write slots 2t apart, 8 banks each
 
+// Dynamic shared memory of the tiles of nslots tables, up to 32 KB.  With the
+// 19 KB of static buffers, 30 tiles (233 tables) and more pass the 48 KB that a
+// kernel gets without asking: cas_estimator_create asks.
+constexpr size_t eval_tile_smem(int nslots)
+{
+    return sizeof(uint32_t) * kTileWords * ((nslots + kTileLists - 1) / kTileLists);
+}
+
 __global__ void __launch_bounds__(kTileThreads, 4) eval_tile_kernel(const uint32_t* __restrict__ tiles, uint32_t high,
                                                                     const int64_t* __restrict__ toff, int nslots,
                                                                     const float* __restrict__ tables, int64_t T,
@@ -515,7 +523,11 @@ CAS_API cas_status cas_estimator_create(const uint64_t* masks, int n_masks, int 
     CAS_TRY(upload(&e->d_inst0, inst0));
     CAS_TRY(upload(&e->d_itables0, e->ps_stored.tables));
     CAS_TRY(upload(&e->d_first, first));
-    if (tiled) CAS_TRY(upload(&e->d_tiles, tiles));
+    if (tiled) {
+        CAS_TRY(upload(&e->d_tiles, tiles));
+        CAS_CUDA(cudaFuncSetAttribute(eval_tile_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      static_cast<int>(eval_tile_smem(kMaxSlots))));
+    }
     const int64_t total = static_cast<int64_t>(e->stages) * e->T;
     CAS_CUDA(dmalloc(&e->d_tables, sizeof(float) * std::max<int64_t>(total, 1)));
     cudaStream_t s = static_cast<cudaStream_t>(stream);
@@ -576,10 +588,10 @@ CAS_API cas_status cas_estimator_eval(const cas_estimator* e, const uint64_t* d_
     const auto* pos = reinterpret_cast<const ulonglong2*>(d_positions);
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     if (e->d_tiles) {
-        const size_t smem = sizeof(uint32_t) * kTileWords * ((nslots + kTileLists - 1) / kTileLists);
         const unsigned grid = static_cast<unsigned>(std::min<int64_t>((n + kTileThreads - 1) / kTileThreads, 4LL * sm_count()));
-        { eval_tile_kernel<<<grid, kTileThreads, smem, s>>>(e->d_tiles, e->high_tiles, e->d_toff, nslots, e->d_tables,
-                                                            e->T, e->stage_size, e->stages, pos, n, d_scores); cas::count_launch(); }
+        { eval_tile_kernel<<<grid, kTileThreads, eval_tile_smem(nslots), s>>>(
+            e->d_tiles, e->high_tiles, e->d_toff, nslots, e->d_tables, e->T, e->stage_size, e->stages, pos, n,
+            d_scores); cas::count_launch(); }
     } else {
         { eval_kernel<<<grid_of(n), 256, 0, s>>>(e->d_slots, nslots, e->d_tables, e->T, e->stage_size, e->stages, pos,
                                                  n, d_scores); cas::count_launch(); }
