@@ -59,6 +59,16 @@ cudaError_t hmalloc(T** p, size_t bytes)
     return hmalloc_bytes(reinterpret_cast<void**>(p), bytes);
 }
 
+// Scratch of a call that does not wait: allocated and freed in the order of
+// the stream s, from a pool of the library's own (memory.cu).  May be captured.
+cudaError_t smalloc_bytes(void** p, size_t bytes, cudaStream_t s);
+void sfree(void* p, cudaStream_t s);
+template <typename T>
+cudaError_t smalloc(T** p, size_t bytes, cudaStream_t s)
+{
+    return smalloc_bytes(reinterpret_cast<void**>(p), bytes, s);
+}
+
 }  // namespace cas
 
 // Returns from the enclosing cas_status function on a CUDA error.

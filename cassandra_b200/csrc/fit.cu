@@ -85,13 +85,12 @@ CAS_API cas_status cas_generate_positions(uint64_t seed, int64_t n, int min_empt
     CAS_TRY(require_device());
     if (n == 0) return CAS_OK;
     auto s = static_cast<cudaStream_t>(stream);
-    // from the library's cache: an empty stream-ordered pool maps memory for
-    // these four bytes, at 0.1 to 10 ms a call
     struct Flag {
         unsigned int* p = nullptr;
-        ~Flag() { dfree(p); }
-    } flag;
-    CAS_CUDA(dmalloc(&flag.p, sizeof(unsigned int)));
+        cudaStream_t s;
+        ~Flag() { sfree(p, s); }
+    } flag{nullptr, s};
+    CAS_CUDA(smalloc(&flag.p, sizeof(unsigned int), s));
     unsigned int* fails = flag.p;
     CAS_CUDA(cudaMemsetAsync(fails, 0, sizeof(unsigned int), s));
     { generate_positions_kernel<<<grid(n), 256, 0, s>>>(seed, n, min_empties, max_empties,
@@ -135,22 +134,14 @@ CAS_API cas_status cas_generate_targets_rows(const cas_csr* a, uint64_t seed, do
     CAS_REQUIRE(a && (d_b || a->rows == 0) && first_row >= 0, CAS_ERR_INVALID_ARGUMENT,
                 "cas_generate_targets: bad argument");
     auto s = static_cast<cudaStream_t>(stream);
-    double* w = d_w_true;
-    // from the library's cache (which hands the block out again only after
-    // the device has been waited for), from the stream's pool under capture
-    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-    CAS_CUDA(cudaStreamIsCapturing(s, &cap));
-    const size_t w_bytes = sizeof(double) * std::max<int64_t>(a->cols, 1);
+    // the call only enqueues work, so its scratch lives in the stream's order
     struct Weights {
         double* p = nullptr;
-        ~Weights() { dfree(p); }
-    } cached;
-    if (!w && cap == cudaStreamCaptureStatusNone) {
-        CAS_CUDA(dmalloc(&cached.p, w_bytes));
-        w = cached.p;
-    } else if (!w) {
-        CAS_CUDA(cudaMallocAsync(&w, w_bytes, s));
-    }
+        cudaStream_t s;
+        ~Weights() { sfree(p, s); }
+    } own{nullptr, s};
+    if (!d_w_true) CAS_CUDA(smalloc(&own.p, sizeof(double) * std::max<int64_t>(a->cols, 1), s));
+    double* w = d_w_true ? d_w_true : own.p;
     { true_weights_kernel<<<grid(a->cols), 256, 0, s>>>(seed, a->cols, w_sigma, w); cas::count_launch(); }
     CAS_CHECK_LAUNCH();
     if (a->rows) {
@@ -159,7 +150,6 @@ CAS_API cas_status cas_generate_targets_rows(const cas_csr* a, uint64_t seed, do
         { targets_kernel<<<grid(a->rows), 256, 0, s>>>(d_b, a->rows, seed, noise_sigma, first_row, d_b); cas::count_launch(); }
         CAS_CHECK_LAUNCH();
     }
-    if (!d_w_true && !cached.p) cudaFreeAsync(w, s);
     return CAS_OK;
 }
 

@@ -66,7 +66,9 @@ CAS_API long long cas_kernel_launches(void);
  * from a per-device cache that keeps freed blocks for the next object of a
  * similar size (the training loop fits the same shapes repeatedly), up to a
  * quarter of the device's memory.  A cached block is reused only after the
- * work that used it has finished, as with cudaFree.
+ * work that used it has finished, as with cudaFree.  Calls that only enqueue
+ * work (cas_generate_targets) take scratch in their stream's order from a pool
+ * of the library's own that keeps at most 64 MB and counts as cached.
  * cas_cached_memory: bytes held in the cache now (free, not in use).
  * cas_release_cached_memory: returns every cached block to the driver. */
 CAS_API size_t cas_cached_memory(void);
@@ -423,7 +425,8 @@ CAS_API cas_status cas_generate_positions_host(uint64_t seed, int64_t first, int
                                                int max_empties, uint64_t* h_out);
 /* Targets b = clamp(2*rint((A w* + e)/2), -64, 64) with w* ~ N(0, w_sigma^2)
  * per column and e ~ N(0, noise_sigma^2) per row, seeded.  Optionally
- * returns w* (cols doubles, may be NULL). */
+ * returns w* (cols doubles, may be NULL).  Enqueued on the stream, without a
+ * wait; it may be captured. */
 CAS_API cas_status cas_generate_targets(const cas_csr* a, uint64_t seed, double w_sigma, double noise_sigma,
                                         double* d_b, double* d_w_true, void* stream);
 /* The same targets for a block of rows of a larger system: row r of `a` is
