@@ -1447,7 +1447,7 @@ struct AtyShared {
     int64_t out;             // offset of its partials
     const T* yb;             // y of its first block
     int b0, nblk;
-    int left;                // rows of the problem from its first block on
+    int full, rest;          // blocks from the first one on that are whole (at most nblk), rows of the next one
     int pc0, npc;            // its pieces
     int2 share[kMaxPieces];  // columns of the unit in each piece
     int unit;                // the CTA's next unit (persistent schedules)
@@ -1505,9 +1505,12 @@ __device__ __forceinline__ void aty_item(const FastGeometry& g, const TView& tv,
         const int q = g.prob_of_block(b0);  // items never span problems
         if (pdone && pdone[q]) return;      // retired problem: partials unused
         const int64_t row0 = g.prow0[q] + static_cast<int64_t>(b0 - g.pblk0[q]) * kBlockRows;
-        const int left = static_cast<int>(g.prow0[q + 1] - row0);
+        // the problem's rows from here on: 2^31 and more with one entry a row
+        const int64_t left = g.prow0[q + 1] - row0;
+        const int full = static_cast<int>(min(left / kBlockRows, static_cast<int64_t>(b1 - b0)));
+        const int rest = static_cast<int>(left % kBlockRows);
         const T* yb = y ? y + (row0 - g.block_row0(y_block0)) : nullptr;
-        stage_y(yb, min(left, kBlockRows), ytile);
+        stage_y(yb, full > 0 ? kBlockRows : rest, ytile);
         if (warp == 0) {
             const int pc0 = sh.sc_piece0[sc], npc = sh.sc_piece0[sc + 1] - pc0;
             if (threadIdx.x == 0) {
@@ -1515,7 +1518,8 @@ __device__ __forceinline__ void aty_item(const FastGeometry& g, const TView& tv,
                 sh.yb = yb;
                 sh.b0 = b0;
                 sh.nblk = b1 - b0;
-                sh.left = left;
+                sh.full = full;
+                sh.rest = rest;
                 sh.pc0 = pc0;
                 sh.npc = npc;
             }
@@ -1533,12 +1537,12 @@ __device__ __forceinline__ void aty_item(const FastGeometry& g, const TView& tv,
         if (i > 0) {
             __syncthreads();  // the tile is free
             stage_y(sh.yb ? sh.yb + static_cast<int64_t>(i) * kBlockRows : nullptr,
-                    min(sh.left - i * kBlockRows, kBlockRows), ytile);
+                    i < sh.full ? kBlockRows : sh.rest, ytile);
         }
         if (i + 1 < sh.nblk) {
             if (sh.yb)  // the next block's y slice into L2
                 prefetch_l2(sh.yb + static_cast<int64_t>(i + 1) * kBlockRows,
-                            min(sh.left - (i + 1) * kBlockRows, kBlockRows) * static_cast<int64_t>(sizeof(T)));
+                            (i + 1 < sh.full ? kBlockRows : sh.rest) * static_cast<int64_t>(sizeof(T)));
             if (warp == 0) {  // and its table, a block ahead
                 fill_pieces(g, sh.pm + sh.pc0, sh.npc, sub_start, sh.share, sh.b0 + i + 1, sh.bp[(i + 1) & 1]);
                 if (!STRETCH) prefetch_first_rounds(g32, sh.bp[(i + 1) & 1]);
