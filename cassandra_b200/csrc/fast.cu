@@ -1990,7 +1990,7 @@ cas_status build_items(const FastGeometry& g, const std::vector<int64_t>& entrie
     std::vector<int> item_sc, item_b0, item_b1, sc_item0;
     std::vector<int64_t> item_part;
     int64_t part_elems = 0;
-    if (range_major && g.nprob == 1 && nsc > 1) {
+    if (range_major && g.nprob == 1 && nsc > 1 && g.nblocks > 0) {
         // One fit: every super-chunk shares one partition of the blocks into
         // ranges, and the items run range by range (within a range the
         // heaviest super-chunks first), so that the CTAs at work at one time
@@ -2486,6 +2486,11 @@ cas_status fast_build(const DevicePatterns& dp, const PatternSet& ps, const uint
         CAS_TRY(build_items(g, entries, 1, 2, true, true, false, sizeof(double), f.t64));
         if (g.nprob == 1) CAS_TRY(build_block_items(g, f.tb));  // evaluator minibatches: single fits only
         if (diag_int && rows > 0) CAS_TRY(fast_diag(f, diag_int, s));
+    } else {
+        // no items, but the column sums of a solve read the lists' tables
+        const Sched& c = kSchedDefault;
+        CAS_TRY(build_items(g, entries, c.per_sc, c.ips, c.range_major, c.pack, c.persistent, sizeof(float), f.t32));
+        CAS_TRY(build_items(g, entries, 1, 2, false, true, false, sizeof(double), f.t64));
     }
     return CAS_OK;
 }
