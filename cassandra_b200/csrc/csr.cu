@@ -430,45 +430,56 @@ __global__ void bound_check_kernel(const uint32_t* __restrict__ idx, int64_t n, 
 // Products.
 // ---------------------------------------------------------------------------
 
-// y = A x: a warp takes kSpmvRows rows at a time, its lanes stride over each
-// row's K indices (coalesced 4K-byte streams), gathers of x summed in FP64,
+// y = A x: a warp takes ROWS rows at a time, its lanes stride over each row's K
+// indices (coalesced 4K-byte streams), gathers of x summed in FP64,
 // warp-shuffle trees.  Bound by the gathers' L1 lookups, one line a cycle and
 // SM (2M rows of 32 at random: 227 us), once the rows' chains of index, gather
 // and tree overlap: a row at a time 281 us (FP64 307), four 237 (261).  A part
 // of x in shared memory (64 to 180 KB, one CTA an SM) took 281 to 482.
+//
+// A row of more than kSpmvShortRow entries has loads enough in flight by
+// itself, and four of them are a chain as long as the kernel when rows are few:
+// us, FP32, a row at a time and four: 148 rows of 8,192 50 and 366, 5,000 of
+// 3,000 88 and 156, 60,000 of 1,000 98 and 147, 30,000 of 100 29 and 32; the
+// other way 300,000 of 100 146 and 138, 100,000 of 8 27 and 23.
 constexpr int kSpmvRows = 4;
+constexpr int kSpmvShortRow = 64;
 
-template <typename T>
+template <typename T, int ROWS>
 __global__ void __launch_bounds__(256) spmv_kernel(const uint32_t* __restrict__ idx, int64_t rows, int k,
                                                    const T* __restrict__ x, T* __restrict__ y)
 {
     const int lane = threadIdx.x & 31;
     const int64_t warps = static_cast<int64_t>(gridDim.x) * (blockDim.x >> 5);
-    for (int64_t r = (static_cast<int64_t>(blockIdx.x) * (blockDim.x >> 5) + (threadIdx.x >> 5)) * kSpmvRows; r < rows;
-         r += warps * kSpmvRows) {
+    for (int64_t r = (static_cast<int64_t>(blockIdx.x) * (blockDim.x >> 5) + (threadIdx.x >> 5)) * ROWS; r < rows;
+         r += warps * ROWS) {
         const uint32_t* row = idx + r * k;
-        const int n = static_cast<int>(min(rows - r, static_cast<int64_t>(kSpmvRows)));
-        double acc[kSpmvRows] = {};
-        for (int j = lane; j < k; j += 32) {
-            uint32_t c[kSpmvRows];
-            T v[kSpmvRows];
+        const int n = static_cast<int>(min(rows - r, static_cast<int64_t>(ROWS)));
+        double acc[ROWS] = {};
+        if constexpr (ROWS == 1) {
+            for (int j = lane; j < k; j += 32) acc[0] += static_cast<double>(__ldg(x + __ldg(row + j)));
+        } else {
+            for (int j = lane; j < k; j += 32) {
+                uint32_t c[ROWS];
+                T v[ROWS];
 #pragma unroll
-            for (int i = 0; i < kSpmvRows; i++)
-                if (i < n) c[i] = __ldg(row + static_cast<int64_t>(i) * k + j);
+                for (int i = 0; i < ROWS; i++)
+                    if (i < n) c[i] = __ldg(row + static_cast<int64_t>(i) * k + j);
 #pragma unroll
-            for (int i = 0; i < kSpmvRows; i++)
-                if (i < n) v[i] = __ldg(x + c[i]);
+                for (int i = 0; i < ROWS; i++)
+                    if (i < n) v[i] = __ldg(x + c[i]);
 #pragma unroll
-            for (int i = 0; i < kSpmvRows; i++)
-                if (i < n) acc[i] += static_cast<double>(v[i]);
+                for (int i = 0; i < ROWS; i++)
+                    if (i < n) acc[i] += static_cast<double>(v[i]);
+            }
         }
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1)
 #pragma unroll
-            for (int i = 0; i < kSpmvRows; i++) acc[i] += __shfl_xor_sync(0xffffffffu, acc[i], o);
+            for (int i = 0; i < ROWS; i++) acc[i] += __shfl_xor_sync(0xffffffffu, acc[i], o);
         double mine = acc[0];
 #pragma unroll
-        for (int i = 1; i < kSpmvRows; i++)
+        for (int i = 1; i < ROWS; i++)
             if (lane == i) mine = acc[i];
         if (lane < n) y[r + lane] = static_cast<T>(mine);
     }
@@ -525,7 +536,9 @@ template <typename T>
 cas_status spmv(const CsrView& a, const T* x, T* y, cudaStream_t s)
 {
     if (a.rows == 0) return CAS_OK;
-    { spmv_kernel<T><<<grid_for(a.rows, 8 * kSpmvRows), 256, 0, s>>>(a.idx, a.rows, a.k, x, y); cas::count_launch(); }
+    const bool several = a.k <= kSpmvShortRow;
+    auto kernel = several ? spmv_kernel<T, kSpmvRows> : spmv_kernel<T, 1>;
+    { kernel<<<grid_for(a.rows, several ? 8 * kSpmvRows : 8), 256, 0, s>>>(a.idx, a.rows, a.k, x, y); cas::count_launch(); }
     CAS_CHECK_LAUNCH();
     return CAS_OK;
 }
