@@ -653,12 +653,12 @@ __device__ __forceinline__ void gather_words(const uint4& u, int slots, const T*
     }
 }
 
-constexpr int kRowPatterns = 8;  // patterns whose index words a thread holds at once
+constexpr int kRowPatterns = 8;  // most patterns whose index words a thread holds at once
 
-// Row r of block blk times x: every index word first, then the gathers, so
-// that they are in flight together.  TABLE: the patterns of tab have their
-// slice of x in table.
-template <typename T, bool ALL8, bool TABLE>
+// Row r of block blk times x: the index words of AHEAD patterns first, then
+// their gathers, so that they are in flight together.  TABLE: the patterns of
+// tab have their slice of x in table.
+template <typename T, bool ALL8, bool TABLE, int AHEAD = kRowPatterns>
 __device__ __forceinline__ typename AccOf<T>::type row_sum(const FastGeometry& g, const uint16_t* __restrict__ a16,
                                                            int64_t blk, int r, const T* __restrict__ x,
                                                            const FastTable& tab, const T* __restrict__ table)
@@ -666,10 +666,10 @@ __device__ __forceinline__ typename AccOf<T>::type row_sum(const FastGeometry& g
     const uint16_t* bp = a16 + blk * static_cast<int64_t>(kBlockRows) * g.k;
     const int pad = static_cast<int>(g.padded_rows(blk));
     typename AccOf<T>::type acc = 0;
-    for (int p0 = 0; p0 < g.npat; p0 += kRowPatterns) {
-        uint4 w[kRowPatterns];
+    for (int p0 = 0; p0 < g.npat; p0 += AHEAD) {
+        uint4 w[AHEAD];
 #pragma unroll
-        for (int i = 0; i < kRowPatterns; i++) {
+        for (int i = 0; i < AHEAD; i++) {
             const int p = p0 + i;
             if (p < g.npat) {
                 const int ns = ALL8 ? 8 : g.slots[p];
@@ -677,7 +677,7 @@ __device__ __forceinline__ typename AccOf<T>::type row_sum(const FastGeometry& g
             }
         }
 #pragma unroll
-        for (int i = 0; i < kRowPatterns; i++) {
+        for (int i = 0; i < AHEAD; i++) {
             const int p = p0 + i;
             if (p < g.npat) {
                 const int ns = ALL8 ? 8 : g.slots[p];
@@ -1653,25 +1653,39 @@ __global__ void __launch_bounds__(kFastThreads, 1) fast_spmv_t_kernel(FastGeomet
 // Evaluator forward on a row range: score[r - row0] = sum_j w[col_rj], one
 // thread per row (row_sum), gathers of w through L1/L2 (the range is a
 // minibatch, too short to amortise staging w in shared memory).
-constexpr int kEvalRows = 128;  // threads of a CTA
+//
+// How many patterns' index words a thread loads ahead of its gathers depends
+// on what a range is bound by.  Rows that are resident at once are bound by
+// their chains of loads: all words ahead.  Longer ranges are bound by the
+// gathers' L1 lookups and want as many warps as possible: a pattern at a time,
+// in few registers (all words ahead leave 7 CTAs an SM).  Forward, us, all
+// words ahead and a pattern at a time: eight expanded patterns, 16,384 rows 9.4
+// and 11.6, 131,072 15.0 and 15.5, 163,840 26.3 and 17.2, 3.9M 330 and 290.
+// Without the expanded layout's 8 slots everywhere the loads ahead are
+// predicated and pay less: the forward takes a pattern at a time (five reference
+// patterns, 16,384 rows 9.0 and 8.3, 3.9M 169 and 115), the loss kernel four
+// (1, 4 and 8 ahead: 16,384 rows 11.0, 7.0, 6.7; 3.9M 137, 126, 141).
+constexpr int kEvalRows = 128;                      // threads of a CTA
+constexpr int kEvalCtas = 28;                       // most CTAs per SM of a launch
+constexpr int64_t kEvalResident = 7 * kEvalRows;    // rows per SM at once with all words ahead
 
-template <bool ALL8>
+template <bool ALL8, int AHEAD>
 __device__ __forceinline__ float eval_row(const FastGeometry& g, const uint16_t* __restrict__ a16,
                                           const float* __restrict__ w, int64_t r)
 {
     int64_t b, rb;
     g.locate_row(r, b, rb);
-    return row_sum<float, ALL8, false>(g, a16, b, static_cast<int>(rb), w + g.col_base(b), FastTable{}, nullptr);
+    return row_sum<float, ALL8, false, AHEAD>(g, a16, b, static_cast<int>(rb), w + g.col_base(b), FastTable{}, nullptr);
 }
 
-template <bool ALL8>
+template <bool ALL8, int AHEAD>
 __global__ void __launch_bounds__(kEvalRows) fast_rows_forward_kernel(FastGeometry g, const uint16_t* __restrict__ a16,
                                                                       const float* __restrict__ w, int64_t row0,
                                                                       int64_t row1, float* __restrict__ out)
 {
     for (int64_t r = row0 + static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; r < row1;
          r += static_cast<int64_t>(gridDim.x) * blockDim.x)
-        out[r - row0] = eval_row<ALL8>(g, a16, w, r);
+        out[r - row0] = eval_row<ALL8, AHEAD>(g, a16, w, r);
 }
 
 // Dense column sums of per-block partials laid out [block][cols].
@@ -1689,10 +1703,8 @@ __global__ void block_partial_sum_kernel(const float* __restrict__ partial, int 
 // Forward of a training step fused with its loss: per row the score (as in
 // fast_rows_forward_kernel), d = score - target, the Huber loss of d summed
 // per CTA into red[blockIdx.x] (FP64, deterministic tree), and the loss
-// gradient dscore = clamp(d, -delta, delta) / n for the adjoint.  Bound by
-// latency: a row's index words are all loaded before its gathers (65,536 rows
-// of eight expanded patterns: 13.1 us pattern by pattern, 9.6 us so).
-template <bool ALL8>
+// gradient dscore = clamp(d, -delta, delta) / n for the adjoint.
+template <bool ALL8, int AHEAD>
 __global__ void __launch_bounds__(kEvalRows) eval_loss_grad_kernel(FastGeometry g, const uint16_t* __restrict__ a16,
                                                                    const float* __restrict__ w,
                                                                    const float* __restrict__ target, int64_t row0,
@@ -1704,7 +1716,7 @@ __global__ void __launch_bounds__(kEvalRows) eval_loss_grad_kernel(FastGeometry 
     for (int64_t r = row0 + static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; r < row1;
          r += static_cast<int64_t>(gridDim.x) * blockDim.x) {
         const float tg = target[r - row0];
-        const float d = eval_row<ALL8>(g, a16, w, r) - tg;
+        const float d = eval_row<ALL8, AHEAD>(g, a16, w, r) - tg;
         const float ad = fabsf(d);
         hs += ad < delta ? 0.5f * d * d : delta * (ad - 0.5f * delta);
         dscore[r - row0] = fminf(fmaxf(d, -delta), delta) * inv_n;
@@ -2636,12 +2648,22 @@ cas_status fast_spmv_t(const FastLayout& f, const T* y, T* x, cudaStream_t s)
     return CAS_OK;
 }
 
+static bool eval_resident(int64_t n) { return n <= kEvalResident * sm_count(); }
+static unsigned eval_grid(int64_t n)
+{
+    return static_cast<unsigned>(std::min<int64_t>(
+        {(n + kEvalRows - 1) / kEvalRows, static_cast<int64_t>(kEvalCtas) * sm_count(), int64_t(kEvalRedMax)}));
+}
+
 cas_status fast_eval_forward(const FastLayout& f, int64_t row0, int64_t row1, const float* w, float* score,
                              cudaStream_t s)
 {
     if (row1 <= row0) return CAS_OK;
-    auto kernel = all_slots_8(f.g) ? fast_rows_forward_kernel<true> : fast_rows_forward_kernel<false>;
-    { kernel<<<fgrid(row1 - row0, kEvalRows) * 4, kEvalRows, 0, s>>>(f.g, f.a16, w, row0, row1, score); cas::count_launch(); }
+    const int64_t n = row1 - row0;
+    auto kernel = !all_slots_8(f.g) ? fast_rows_forward_kernel<false, 1>
+                                    : (eval_resident(n) ? fast_rows_forward_kernel<true, kRowPatterns>
+                                                        : fast_rows_forward_kernel<true, 1>);
+    { kernel<<<eval_grid(n), kEvalRows, 0, s>>>(f.g, f.a16, w, row0, row1, score); cas::count_launch(); }
     CAS_CHECK_LAUNCH();
     return CAS_OK;
 }
@@ -2737,8 +2759,10 @@ cas_status fast_eval_adam_step(FastLayout& f, int64_t row0, int64_t row1, const 
     const int64_t b0 = row0 / kBlockRows, b1 = (row1 + kBlockRows - 1) / kBlockRows;
     if (f.g.cols == 0 || n <= 0) return CAS_OK;
     CAS_TRY(eval_buffers(f, b1 - b0, s));
-    const unsigned g1 = std::min<unsigned>(fgrid(n, kEvalRows), kEvalRedMax);
-    auto loss = all_slots_8(f.g) ? eval_loss_grad_kernel<true> : eval_loss_grad_kernel<false>;
+    const unsigned g1 = eval_grid(n);
+    auto loss = !all_slots_8(f.g) ? eval_loss_grad_kernel<false, 4>
+                                  : (eval_resident(n) ? eval_loss_grad_kernel<true, kRowPatterns>
+                                                      : eval_loss_grad_kernel<true, 1>);
     { loss<<<g1, kEvalRows, 0, s>>>(f.g, f.a16, w, target, row0, row1, o.delta, 1.0f / static_cast<float>(n),
                                     f.eval_dscore, f.eval_red); cas::count_launch(); }
     CAS_CHECK_LAUNCH();
