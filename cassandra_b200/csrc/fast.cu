@@ -1939,14 +1939,14 @@ std::vector<int64_t> item_entries(const FastGeometry& g, const std::vector<int64
     return out;
 }
 
-// The splits of every item (fixed cost and entries each) on the GPU: none
-// from kPlanWaves items a CTA on, else those of the best limit.
-std::vector<int> plan_splits(const std::vector<float>& fixed, const std::vector<float>& entries)
+// The splits of n items, each there `copies` times (fixed cost and entries
+// each), on the GPU: none from kPlanWaves items a CTA on, else those of the
+// best limit.
+std::vector<int> plan_splits(const float* fixed, const float* entries, size_t n, size_t copies)
 {
-    const size_t n = fixed.size();
     const float ctas = static_cast<float>(sm_count());
     std::vector<int> K(n, 1);
-    if (n >= static_cast<size_t>(kPlanWaves) * sm_count()) return K;
+    if (n * copies >= static_cast<size_t>(kPlanWaves) * sm_count()) return K;
     float top = 0, best = 0, best_limit = 0;
     for (size_t i = 0; i < n; i++) top = std::max(top, fixed[i] + entries[i]);
     for (int j = 0; j < kPlanLimits; j++) {
@@ -1958,6 +1958,8 @@ std::vector<int> plan_splits(const std::vector<float>& fixed, const std::vector<
             longest = std::max(longest, fixed[i] + entries[i] / static_cast<float>(k));
             units += static_cast<float>(k);
         }
+        units *= static_cast<float>(copies);
+        load *= static_cast<float>(copies);
         const float est = plan_estimate(units, load, longest, ctas);
         if (j == 0 || est < best) {
             best = est;
@@ -1979,7 +1981,7 @@ void pack_units(const std::vector<int>& item_b0, const std::vector<int>& item_b1
         fixed[i] = unit_fixed(fp64, item_b1[i] - item_b0[i]);
         en[i] = static_cast<float>(entries[i]);
     }
-    const std::vector<int> K = plan_splits(fixed, en);
+    const std::vector<int> K = plan_splits(fixed.data(), en.data(), n, 1);
     std::vector<int> order(n);
     for (size_t i = 0; i < n; i++) order[i] = static_cast<int>(i);
     if (n < static_cast<size_t>(kPlanWaves) * sm_count())
@@ -2727,18 +2729,18 @@ static cas_status eval_buffers(FastLayout& f, int64_t nb, cudaStream_t s)
 }
 
 // The adjoint's per-block partials of blocks [b0, b1) on g into eval_partial.
-// One CTA per (block, chunk) item: splitting a minibatch's items over more
-// CTAs re-stages y per split and was measured slower (8.6 against 6.8 ms
-// per epoch of the 8M-row evaluator workload).
+// The (block, chunk) items of a short range are split (plan_splits) by the
+// chunks' mean entries in a block, the same in every block: the plan is made
+// anew in each call, from one block's chunks (4 blocks of eight expanded
+// patterns: the kernel takes 25 us with whole items, 18 so; planned over all
+// items, 24 blocks cost the host 30 us a call).
 static cas_status eval_adjoint_partials(FastLayout& f, int64_t b0, int64_t b1, const float* g, cudaStream_t s)
 {
     const size_t smem = spmv_t_smem<float>(1);
-    // the chunks' splits from their mean entries in a block (a chunk of a
-    // block holds 1% to 100% of a pattern's)
     const int nch = f.g.nchunks;
-    std::vector<float> fixed(static_cast<size_t>((b1 - b0) * nch), unit_fixed(false, 1)), entries(fixed.size());
-    for (size_t i = 0; i < entries.size(); i++) entries[i] = f.chunk_entries[i % nch];
-    const std::vector<int> K = plan_splits(fixed, entries);
+    float fixed[kMaxChunks];
+    std::fill_n(fixed, nch, unit_fixed(false, 1));
+    const std::vector<int> K = plan_splits(fixed, f.chunk_entries, nch, static_cast<size_t>(b1 - b0));
     BlockUnits bu;
     for (int ch = 0; ch < nch; ch++) {
         bu.splits[ch] = static_cast<uint8_t>(K[ch]);
