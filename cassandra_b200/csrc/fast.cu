@@ -1960,6 +1960,11 @@ std::vector<int> plan_splits(const float* fixed, const float* entries, size_t n,
         }
         units *= static_cast<float>(copies);
         load *= static_cast<float>(copies);
+        // items that fit one wave are not cut into two: the second pays the
+        // fixed cost of its units once more, and an SM runs one unit at a time
+        // (us, whole and cut: a training step's 6 blocks of eight reference
+        // patterns 17 and 24, FP64 A'y of 80 blocks of two 64 and 80)
+        if (j > 0 && units > ctas && static_cast<float>(n * copies) <= ctas) break;
         const float est = plan_estimate(units, load, longest, ctas);
         if (j == 0 || est < best) {
             best = est;
