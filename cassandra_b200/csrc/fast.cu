@@ -2364,7 +2364,12 @@ cas_status tune_transpose(FastLayout& f, const std::vector<int64_t>& entries, cu
 }
 
 // The patterns whose slices of x the table kernel keeps in shared memory: by
-// entries a row per column, while they fit.
+// entries a row per column, while they fit, and of those the ones that a CTA
+// gathers from as often as the slice has bytes between two stagings (one per
+// CTA, and one more per problem of a batch).  Below that, staging takes longer
+// than its gathers save: one pattern of 29,646 columns and 4 slots, FP32, us
+// staged and not, 49 blocks 39 and 29, 200 66 and 59, 300 83 and 80; five
+// reference patterns with 65 KB for 10 slots, 49 blocks 56 and 50, 80 68 and 70.
 FastTable table_plan(const FastGeometry& g, size_t elem)
 {
     FastTable t;
@@ -2375,8 +2380,9 @@ FastTable table_plan(const FastGeometry& g, size_t elem)
     });
     for (int p = 0; p < kMaxFastPatterns; p++) t.base[p] = -1;
     const int room = static_cast<int>(kTableBytes / elem);
+    const int64_t rows = g.rows / (sm_count() + g.nprob - 1);  // of a staging
     for (int p : order)
-        if (t.elems + g.space[p] <= room) {
+        if (t.elems + g.space[p] <= room && rows * g.slots[p] >= static_cast<int64_t>(elem) * g.space[p]) {
             t.base[p] = t.elems;
             t.elems += g.space[p];
         }
