@@ -1825,7 +1825,7 @@ __global__ void fast_col_sum_kernel(FastCols fc, const T* __restrict__ partial, 
 {
     for (int64_t c = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; c < fc.g.cols;
          c += static_cast<int64_t>(gridDim.x) * blockDim.x)
-        x[c] = static_cast<T>(fast_col_sum<T>(fc, partial, c));
+        x[c] = static_cast<T>(fast_col_sum<T, 32>(fc, partial, c));
 }
 
 // The small arrays of a work list, gathered on the host and sent to the

@@ -460,7 +460,32 @@ cas_status fast_spmv_t_partials(const FastLayout& f, const T* y, int* done_flag,
 template <typename T>
 FastCols fast_cols(const FastLayout& f);
 
-template <typename T>
+// acc += the next N partials, all loaded before the adds, in their order.  (An
+// unrolled loop leaves it to the compiler how many loads it issues ahead, and
+// it chose otherwise in each kernel: the FP32 LSQR step of one pattern's 148
+// partials a column, 786,432 rows, took 14.5 us instead of 8.8, where the PCG
+// step took 8.2 instead of 10.7; 5.9 and 5.7 so.  Remainders go by halves, as
+// a predicated batch costs as much as a full one.)
+template <typename T, int N>
+__device__ __forceinline__ void sum_ahead(const T*& at, int64_t stride, double& acc)
+{
+    T v[N];
+#pragma unroll
+    for (int u = 0; u < N; u++) {
+        v[u] = *at;
+        at += stride;
+    }
+#pragma unroll
+    for (int u = 0; u < N; u++) acc += static_cast<double>(v[u]);
+}
+
+// Column c of A'y, TOP partials ahead: 32 where the sum is all the kernel does
+// (fast_col_sum_kernel, us, 16 and 32 ahead: FP64, 4.9M rows of two patterns, 148
+// partials a column, 36 and 21; FP32, 9.8M rows of eight expanded ones 24 and
+// 18), 16 where its registers are shared (32 take the steps of the solvers past
+// 64 and a quarter of their CTAs: the PCG step of 786,432 rows of five expanded
+// patterns 8.8 and 12.0).
+template <typename T, int TOP = 16>
 __device__ __forceinline__ double fast_col_sum(const FastCols& fc, const T* partial, int64_t c)
 {
     int64_t q = 0;
@@ -477,16 +502,18 @@ __device__ __forceinline__ double fast_col_sum(const FastCols& fc, const T* part
     const int i0 = fc.sc_item0[sc], n = fc.sc_item0[sc + 1] - i0;
     if (n == 0) return 0;
     // A super-chunk's items have their partials at equal distances, so no
-    // address waits for a load (60 partials a column, 10M rows: 46 -> 39 us;
-    // the PCG update at 4M rows 33 -> 25).  16 loads in flight instead of 8
-    // cost registers: 53 and 28.
+    // address waits for a load.
     const T* at = partial + fc.sc_part[i0] + pos;
     const int64_t stride = n > 1 ? fc.sc_part[i0 + 1] - fc.sc_part[i0] : 0;
     double acc = 0;
-    // unrolled so that the partials' loads are issued ahead of the adds,
-    // which keep their order
-#pragma unroll 8
-    for (int i = 0; i < n; i++) acc += static_cast<double>(at[i * stride]);
+    int left = n;
+    if constexpr (TOP == 32)
+        for (; left >= 32; left -= 32) sum_ahead<T, 32>(at, stride, acc);
+    for (; left >= 16; left -= 16) sum_ahead<T, 16>(at, stride, acc);
+    if (left & 8) sum_ahead<T, 8>(at, stride, acc);
+    if (left & 4) sum_ahead<T, 4>(at, stride, acc);
+    if (left & 2) sum_ahead<T, 2>(at, stride, acc);
+    if (left & 1) sum_ahead<T, 1>(at, stride, acc);
     return acc;
 }
 

@@ -236,6 +236,20 @@ struct ColSum {
         if (kind == 0) return unit_sum(a, unit_partial, c);
         return 0.0;
     }
+    // f(sum) with the sum of this kind alone: a loop over columns inside f is
+    // compiled once per kind, which keeps the loads of a sum together (PCG step
+    // of one pattern, us, with the kinds in one loop and apart: FP32, 4.9M rows
+    // 19.8 and 16.0, FP64 13.1 and 11.5).
+    template <typename F>
+    __device__ __forceinline__ void visit(F&& f) const
+    {
+        if (kind == 1)
+            f([&](int64_t c) { return fast_col_sum<float>(fc, p32, c); });
+        else if (kind == 2)
+            f([&](int64_t c) { return fast_col_sum<double>(fc, p64, c); });
+        else
+            f([&](int64_t c) { return (*this)(c); });
+    }
 };
 
 // ---------------------------------------------------------------------------
@@ -286,17 +300,19 @@ __global__ void __launch_bounds__(kVecThreads) pcg_update_kernel(ColSum cs,
     if (finished(dv.flags)) return;
     const double alpha = dv.scal[kAlpha];
     Comp rz, rr;
-    for (int64_t c = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; c < cs.a.cols;
-         c += static_cast<int64_t>(gridDim.x) * blockDim.x) {
-        const double s = cs(c);
-        x[c] += alpha * p[c];
-        const double rc = r[c] - alpha * s;
-        const double zc = d[c] * rc;
-        r[c] = rc;
-        z[c] = zc;
-        acc_add<COMP>(rz, rc * zc);
-        acc_add<COMP>(rr, rc * rc);
-    }
+    cs.visit([&](auto sum) {
+        for (int64_t c = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; c < cs.a.cols;
+             c += static_cast<int64_t>(gridDim.x) * blockDim.x) {
+            const double s = sum(c);
+            x[c] += alpha * p[c];
+            const double rc = r[c] - alpha * s;
+            const double zc = d[c] * rc;
+            r[c] = rc;
+            z[c] = zc;
+            acc_add<COMP>(rz, rc * zc);
+            acc_add<COMP>(rr, rc * rc);
+        }
+    });
     write_partial<COMP>(part_rz, rz, smem);
     write_partial<COMP>(part_rr, rr, smem);
 }
@@ -530,13 +546,22 @@ __global__ void __launch_bounds__(kVecThreads) lsqr_v_kernel(ColSum cs,
     const double beta = dv.scal[kLBeta];
     const double inv_alpha_prev = dv.scal[kLAlpha] != 0 ? 1.0 / dv.scal[kLAlpha] : 0.0;
     Comp acc;
-    for (int64_t c = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; c < cs.a.cols;
-         c += static_cast<int64_t>(gridDim.x) * blockDim.x) {
-        double val = inv_beta * col_scale(sc, c) * cs(c);
-        if (!init) val -= beta * (v[c] * inv_alpha_prev);
-        v[c] = val;
-        acc_add<COMP>(acc, val * val);
-    }
+    auto columns = [&](const auto& sum) {
+        for (int64_t c = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; c < cs.a.cols;
+             c += static_cast<int64_t>(gridDim.x) * blockDim.x) {
+            double val = inv_beta * col_scale(sc, c) * sum(c);
+            if (!init) val -= beta * (v[c] * inv_alpha_prev);
+            v[c] = val;
+            acc_add<COMP>(acc, val * val);
+        }
+    };
+    // FP64 partials: the kinds in one loop are the faster (eight expanded
+    // patterns, 786,432 rows 8.3 us against 8.5, two patterns 9.8 against 10.5;
+    // FP32 10.2 against 9.3)
+    if constexpr (sizeof(T) == 4)
+        cs.visit(columns);
+    else
+        columns(cs);
     write_partial<COMP>(part, acc, smem);
 }
 
