@@ -725,7 +725,11 @@ __device__ __forceinline__ double store_row(double v, Y* __restrict__ y, const d
 //   8 patterns reference  200 blocks 330 / 420 -> 136 / 166   610: 781 / 1032 -> 371 / 463
 // Up to kAxDirectBlocks blocks the rows are done before a table pays (8
 // patterns expanded, FP32, us without and with it: 16 blocks 26.8 and 28.9,
-// 48 64.1 and 64.0, 74 92.7 and 83).
+// 48 64.1 and 64.0, 74 92.7 and 83).  Of the other sets and FP64 the line lies
+// between 49 and 75 blocks where a table is staged at all (table_plan), and the
+// two are within 5 % of one another there (a call of eight reference patterns,
+// FP32 / FP64, 60 blocks 78 / 87 and 76 / 85, 80 96 / 108 and 87 / 100; five
+// expanded ones, FP64, 60 88.7 and 89.3, 80 108.1 and 106.7).
 //
 // A unit is 1/kAxTableSplit of a block.  part (optional): compensated
 // partials of ||y||^2, one per CTA without act, else per unit laid out
@@ -1450,7 +1454,8 @@ struct AtyShared {
     int sc_piece0[kMaxChunks + 1];
     // the unit: what its loop over blocks needs.  In shared memory, because
     // the reductions need all 64 registers: with these held or spilled, the
-    // FP64 A'y of 610 blocks took 3,020 us, 2,570 so.
+    // FP64 A'y of 610 blocks took 3,020 us, 2,570 so.  (The FP64 reduction
+    // still spills 116 bytes a thread, the FP32 one none.)
     int64_t out;             // offset of its partials
     const T* yb;             // y of its first block
     int b0, nblk;
@@ -1915,7 +1920,6 @@ void pack_pieces(const Pieces& pc, FastTranspose& t, MetaPack& mp)
     t.nsc = static_cast<int>(pc.sc_width.size());
     t.npieces = static_cast<int>(pc.pat.size());
     mp.add(pc.sc_piece0, &t.sc_piece0);
-    mp.add(pc.sc_width, &t.sc_width);
     mp.add(pc.pat, &t.piece_pat);
     mp.add(pc.ch0, &t.piece_ch0);
     mp.add(pc.ch1, &t.piece_ch1);
@@ -1924,9 +1928,6 @@ void pack_pieces(const Pieces& pc, FastTranspose& t, MetaPack& mp)
     mp.add(pc.chunk_acc, &t.chunk_acc);
 }
 
-// Builds the work list of one A'y variant from the entry counts per (block,
-// chunk): super-chunks of at most per_sc chunks of columns, each split into
-// block ranges so that items carry about equal numbers of entries.
 // The G32 entries of every item: its super-chunk's chunks over its blocks.
 std::vector<int64_t> item_entries(const FastGeometry& g, const std::vector<int64_t>& entries_bc, const Pieces& pc,
                                   const std::vector<int>& item_sc, const std::vector<int>& item_b0,
@@ -2007,6 +2008,9 @@ void pack_units(const std::vector<int>& item_b0, const std::vector<int>& item_b1
     mp.add(units, &t.units);
 }
 
+// Builds the work list of one A'y variant from the entry counts per (block,
+// chunk): super-chunks of at most per_sc chunks of columns, each split into
+// block ranges so that items carry about equal numbers of entries.
 cas_status build_items(const FastGeometry& g, const std::vector<int64_t>& entries_bc, int per_sc, int items_per_sm,
                        bool range_major, bool pack, bool persistent, size_t elem, FastTranspose& t)
 {

@@ -166,11 +166,13 @@ struct FastActive {
 // cleared and written: 12,000 cycles), a part per block (y staged, the table,
 // barriers: 8,000) and its entries (280 cycles a round of 1,024 in FP32 and
 // 700 in FP64, which is the shared-memory bandwidth that y gathers and
-// accumulator updates at random banks leave), so it is counted in entries.  With fewer items than kPlanWaves a CTA, the items that cost more
-// than a limit are split; of kPlanLimits limits the one with the shortest
-// estimate is taken.  Items differ by a factor of 100 (the columns of an
-// edge or corner pattern that random play reaches, and those it does not), so
-// a few large ones set the time of a small product that does not split them.
+// accumulator updates at random banks leave), so it is counted in entries.
+// With fewer items than kPlanWaves a CTA, the items that cost more than a limit
+// are split; of kPlanLimits limits the one with the shortest estimate is taken.
+// A list without an active list whose items fit one wave is not split past it
+// (plan_splits).  Items differ by a factor of 100 (the columns of an edge or
+// corner pattern that random play reaches, and those it does not), so a few
+// large ones set the time of a small product that does not split them.
 // A'y of the eight expanded patterns, us, FP32 / FP64, items whole or split by
 // column counts -> these units: 8 blocks 35 / 66 -> 29 / 49, 32 blocks
 // 68 / 199 -> 64 / 156, 64 blocks 126 / 335 -> 117 / 285; a training step's
@@ -226,7 +228,6 @@ struct FastTranspose {
     int nitems = 0;
     int64_t max_item_entries = 0;  // most G32 entries any item reduces
     int* sc_piece0 = nullptr;  // [nsc + 1] first piece of each super-chunk
-    int* sc_width = nullptr;   // [nsc] accumulator columns in use
     int* piece_pat = nullptr;  // [npieces] pattern of the piece
     int* piece_ch0 = nullptr;  // [npieces] first global chunk
     int* piece_ch1 = nullptr;  // [npieces] one past the last global chunk (same pattern)

@@ -58,7 +58,6 @@ TileSet build_tiles(const PatternSet& ps)
         u.kind = in.kind;
         u.slots = static_cast<uint8_t>(slots);
         u.tile0 = static_cast<uint16_t>(tiles - ts.chunk_tile.back());
-        u.pattern = static_cast<uint16_t>(p);
         u.slot0 = static_cast<uint32_t>(s0);
         u.offset = in.offset;
         u.half_size = in.half_size;

@@ -26,7 +26,6 @@ struct IndexUnit {
     uint8_t slots;       // slots of the unit (1..8)
     uint8_t high[2];     // the tile has weights above 255
     uint16_t tile0;      // first tile, counted from the chunk's first
-    uint16_t pattern;
     uint32_t slot0;      // first slot (in the row)
     uint32_t offset;     // column offset of the pattern
     uint32_t half_size, diag_size, table_offset;
