@@ -2377,10 +2377,15 @@ cas_status tune_transpose(FastLayout& f, const std::vector<int64_t>& entries, cu
 // The patterns whose slices of x the table kernel keeps in shared memory: by
 // entries a row per column, while they fit, and of those the ones that a CTA
 // gathers from as often as the slice has bytes between two stagings (one per
-// CTA, and one more per problem of a batch).  Below that, staging takes longer
-// than its gathers save: one pattern of 29,646 columns and 4 slots, FP32, us
-// staged and not, 49 blocks 39 and 29, 200 66 and 59, 300 83 and 80; five
+// CTA, and one more per problem of a batch), or half as often for a slice of up
+// to kTableSmall, which leaves L1 to the others.  Below that, staging takes
+// longer than its gathers save: one pattern of 29,646 columns and 4 slots, FP32,
+// us staged and not, 49 blocks 39 and 29, 200 66 and 59, 300 83 and 80; five
 // reference patterns with 65 KB for 10 slots, 49 blocks 56 and 50, 80 68 and 70.
+// A slice of 26 KB with 2 slots of eight reference patterns, FP64, 92 blocks,
+// saves 4 of 95 us.
+constexpr int kTableSmall = 32 * 1024;
+
 FastTable table_plan(const FastGeometry& g, size_t elem)
 {
     FastTable t;
@@ -2392,11 +2397,13 @@ FastTable table_plan(const FastGeometry& g, size_t elem)
     for (int p = 0; p < kMaxFastPatterns; p++) t.base[p] = -1;
     const int room = static_cast<int>(kTableBytes / elem);
     const int64_t rows = g.rows / (sm_count() + g.nprob - 1);  // of a staging
-    for (int p : order)
-        if (t.elems + g.space[p] <= room && rows * g.slots[p] >= static_cast<int64_t>(elem) * g.space[p]) {
+    for (int p : order) {
+        const int64_t bytes = static_cast<int64_t>(elem) * g.space[p];
+        if (t.elems + g.space[p] <= room && rows * g.slots[p] >= (bytes <= kTableSmall ? bytes / 2 : bytes)) {
             t.base[p] = t.elems;
             t.elems += g.space[p];
         }
+    }
     return t;
 }
 
