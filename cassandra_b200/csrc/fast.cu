@@ -1770,18 +1770,15 @@ __global__ void __launch_bounds__(256) eval_adam_kernel(const float* __restrict_
             wc = w[c];
             mc = m[c];
             vc = v[c];
-            // sixteen partials loaded ahead of their adds, which keep their order
-            // (240 blocks of 105,543 columns: 86 us with one in flight, 34 so)
-            constexpr int kAhead = 16;
+            // the partials ahead of their adds, which keep their order (240
+            // blocks of 105,543 columns: 86 us with one in flight, 34 so)
             const float* at = partial + c;
-            for (int j = 0; j < nb; j += kAhead, at += kAhead * cols) {
-                float part[kAhead];
-#pragma unroll
-                for (int u = 0; u < kAhead; u++) part[u] = j + u < nb ? at[u * cols] : 0.0f;
-#pragma unroll
-                for (int u = 0; u < kAhead; u++)
-                    if (j + u < nb) gc += part[u];
-            }
+            int left = nb;
+            for (; left >= 16; left -= 16) sum_ahead<float, 16>(at, cols, gc);
+            if (left & 8) sum_ahead<float, 8>(at, cols, gc);
+            if (left & 4) sum_ahead<float, 4>(at, cols, gc);
+            if (left & 2) sum_ahead<float, 2>(at, cols, gc);
+            if (left & 1) sum_ahead<float, 1>(at, cols, gc);
         }
         if (!powers) __syncthreads();  // behind the first columns' loads
         powers = true;

@@ -467,8 +467,8 @@ FastCols fast_cols(const FastLayout& f);
 // partials a column, 786,432 rows, took 14.5 us instead of 8.8, where the PCG
 // step took 8.2 instead of 10.7; 5.9 and 5.7 so.  Remainders go by halves, as
 // a predicated batch costs as much as a full one.)
-template <typename T, int N>
-__device__ __forceinline__ void sum_ahead(const T*& at, int64_t stride, double& acc)
+template <typename T, int N, typename Acc>
+__device__ __forceinline__ void sum_ahead(const T*& at, int64_t stride, Acc& acc)
 {
     T v[N];
 #pragma unroll
@@ -477,7 +477,7 @@ __device__ __forceinline__ void sum_ahead(const T*& at, int64_t stride, double& 
         at += stride;
     }
 #pragma unroll
-    for (int u = 0; u < N; u++) acc += static_cast<double>(v[u]);
+    for (int u = 0; u < N; u++) acc += static_cast<Acc>(v[u]);
 }
 
 // Column c of A'y, TOP partials ahead: 32 where the sum is all the kernel does
